@@ -1860,7 +1860,7 @@ int cube_mlp_create(const float *params, int32_t batch_cap, cube_mlp **out) {
     if (ok && cudaMalloc((void **)ptr, bytes) != cudaSuccess) ok = false;
   };
   al(&p.master, sizeof(float) * kMlpParams);
-  al(&p.grad, sizeof(float) * kMlpParams);
+  al(&p.grad, kMlpGradBytes);
   al(&p.mom, sizeof(float) * kMlpParams);
   al(&p.vel, sizeof(float) * kMlpParams);
   al(&p.wb, sizeof(__nv_bfloat16) * kMlpWbElems);
@@ -1885,7 +1885,7 @@ int cube_mlp_create(const float *params, int32_t batch_cap, cube_mlp **out) {
   if (ok) ok = cudaMemcpy(p.master, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice) == cudaSuccess;
   if (ok) ok = cudaMemset(p.mom, 0, sizeof(float) * kMlpParams) == cudaSuccess &&
                cudaMemset(p.vel, 0, sizeof(float) * kMlpParams) == cudaSuccess &&
-               cudaMemset(p.grad, 0, sizeof(float) * kMlpParams) == cudaSuccess;
+               cudaMemset(p.grad, 0, kMlpGradBytes) == cudaSuccess;
   if (ok) {
     launch_mlp_pack(p, g.stream);
     ok = cudaStreamSynchronize(g.stream) == cudaSuccess;

@@ -311,6 +311,9 @@ __host__ __device__ constexpr int mlp_woff(int l) {
 __host__ __device__ constexpr int mlp_boff(int l) { return mlp_woff(l) + mlp_N(l) * mlp_K(l); }
 __host__ __device__ constexpr int mlp_wboff(int l) { return l == 0 ? 0 : mlp_wboff(l - 1) + mlp_Np(l - 1) * mlp_K(l - 1); }
 constexpr int kMlpParams = mlp_boff(3) + kMlpOut;
+// the gradient buffer: one float per parameter, then (8-byte aligned) the FP64 sums of the bias gradients
+constexpr int kMlpGradBias = (kMlpParams + 1) / 2 * 2;
+constexpr size_t kMlpGradBytes = sizeof(float) * kMlpGradBias + sizeof(double) * (3 * kMlpW + kMlpOut);
 constexpr int kMlpWbElems = mlp_wboff(3) + kMlpOutPad * kMlpW;
 
 struct MlpParams {

@@ -803,14 +803,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_apply_tc(MlpApplyK p, int
 }
 
 // ---------------------------------------------------------------------------------------------
-// training GEMM on the 5th-generation tensor cores: C[M][N] = A[M][K] B[N][K]^T + bias[N] with the
+// GEMM of the forward pass (cube_mlp_forward) on the 5th-generation tensor cores: C[M][N] = A[M][K] B[N][K]^T + bias[N] with the
 // epilogue of k_gemm_nt (Z in FP32, H = act(Z) in BF16).  One warpgroup per CTA and a 128-row tile
 // of C (UMMA M = 128, one TMEM lane per row); the CTA's N columns (a multiple of 16, at most 128)
 // accumulate in TMEM.  K advances 64 at a time through two shared-memory stages: the loads of a
 // stage (cp.async, 16 bytes, into the K-major core-matrix layout) overlap the MMAs of the other,
 // whose tcgen05.commit to the stage's mbarrier frees it.  Rows of A past M and of B past N are
-// zero-filled.  K % 16 == 0, lda % 8 == 0, ldb % 8 == 0.  With gridDim.z > 1 (the weight gradients,
-// K = the batch) each CTA takes a slice of K and adds its partial sums to Z (zeroed by the caller).
+// zero-filled.  K % 16 == 0, lda % 8 == 0, ldb % 8 == 0.
 constexpr int kGtM = 128, kGtN = 128, kGtK = 64;
 constexpr size_t kGtStageA = (size_t)kGtM * kGtK * 2, kGtStageB = (size_t)kGtN * kGtK * 2;
 constexpr size_t kGtSmem = 2 * (kGtStageA + kGtStageB) + 2 * 8 + 16;
@@ -843,10 +842,7 @@ __global__ void __launch_bounds__(kGtM, 1) k_gemm_nt_tc(const bf16 *__restrict__
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t idesc = umma_idesc(nt);
-  // this CTA's K slice, whole steps of kGtK
-  const int steps = (K + kGtK - 1) / kGtK, per = (steps + gridDim.z - 1) / gridDim.z;
-  const int kbeg = blockIdx.z * per * kGtK, kend = min(K, kbeg + per * kGtK);
-  const int nk = kend > kbeg ? (kend - kbeg + kGtK - 1) / kGtK : 0;
+  const int nk = (K + kGtK - 1) / kGtK;  // steps of kGtK
   uint32_t phase[2] = {0u, 0u};
   bool ok = true;
   int pending = 0;  // stages with an MMA not yet waited for (bit per stage)
@@ -860,7 +856,7 @@ __global__ void __launch_bounds__(kGtM, 1) k_gemm_nt_tc(const bf16 *__restrict__
       ok = __syncthreads_and(ok);
       if (!ok) break;
     }
-    const int k0 = kbeg + ks * kGtK, kc = min(kGtK, kend - k0);  // kc: a multiple of 16
+    const int k0 = ks * kGtK, kc = min(kGtK, K - k0);  // kc: a multiple of 16
     // A: 128 rows x kc / 8 chunks; B: nt rows x kc / 8 chunks
     for (int i = tid; i < kGtM * (kc / 8); i += kGtM) {
       const int r = i / (kc / 8), c = i % (kc / 8);
@@ -903,7 +899,6 @@ __global__ void __launch_bounds__(kGtM, 1) k_gemm_nt_tc(const bf16 *__restrict__
     // epilogue: thread = row m0 + tid (TMEM lane), 16 columns at a time
     const uint32_t lane_base = (uint32_t)(32 * warp) << 16;
     const int r = m0 + tid;
-    const bool split = gridDim.z > 1;
     for (int c0 = 0; c0 < nt; c0 += 16) {
       float v[16];
       tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
@@ -912,10 +907,6 @@ __global__ void __launch_bounds__(kGtM, 1) k_gemm_nt_tc(const bf16 *__restrict__
         for (int j = 0; j < 16; j++) {
           const int c = n0 + c0 + j;
           if (c >= N) continue;
-          if (split) {
-            atomicAdd(Z + (int64_t)r * ldz + c, v[j]);
-            continue;
-          }
           const float z = v[j] + (bias ? bias[c] : 0.f);
           if (Z) Z[(int64_t)r * ldz + c] = z;
           if (H) H[(int64_t)r * ldh + c] = __float2bfloat16_rn(act ? gelu_f(z) : z);
@@ -930,6 +921,308 @@ __global__ void __launch_bounds__(kGtM, 1) k_gemm_nt_tc(const bf16 *__restrict__
   if (warp == 0) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// One training step's forward and backward pass in one kernel on tcgen05: a CTA takes 128 rows of
+// the batch through all layers and adds its part of every gradient to memory.
+//
+// The separate GEMMs, transposes, GELU passes and column sums took 660 us a step at batch 8192 (28 launches,
+// 543 us of it in the column sums of four blocks each); every intermediate made a round trip through
+// memory.  Here the pre-activations z1..z3 stay in tensor memory (3 x 128 columns in FP32; the
+// other 128 columns take the products that are read at once), the activations in shared memory in the
+// two layouts that the products need: row-major over features (A of the next layer; one
+// buffer, overwritten layer by layer) and transposed (the weight gradients contract over the rows).
+// The weights pass through two buffers, the next matrix arriving by cp.async while a layer runs.
+// What bounds it: 64 CTAs at batch 8192, each a serial chain of 4 + 7 products and their epilogues.
+//   TMEM columns: [0, 384) z1 z2 z3, [384, 512) products read at once (y, da); dW goes to z3's once dz3 is formed.
+constexpr int kTrThreads = 256;  // two warpgroups: thread (row m, half h) takes half of a row's columns
+constexpr size_t kTrWB0 = 0, kTrWB1 = kTcW, kTrW4 = 2 * kTcW, kTrW4t = kTrW4 + kTcW4, kTrXT = kTrW4t + kTcW4,
+                 kTrA1T = kTrXT + (size_t)kMlpK1 * kTcRows * 2, kTrA2T = kTrA1T + kTcAct, kTrA3T = kTrA2T + kTcAct,
+                 kTrAct = kTrA3T + kTcAct, kTrBias = kTrAct + kTcAct,
+                 kTrBar = kTrBias + sizeof(float) * (3 * kMlpW + kMlpOutPad), kTrSmem = kTrBar + 16;
+static_assert(kTrSmem <= 227 * 1024, "one CTA's shared memory");
+
+struct MlpTrainK {
+  const bf16 *X;
+  const float *T;
+  const int32_t *rows;
+  int batch;
+  const bf16 *wb, *wt;
+  const float *master;
+  float *grad;   // zeroed: weight gradients are added here
+  double *gbias;  // zeroed [3 * kMlpW + kMlpOut]: bias gradients
+  float *loss;
+  int32_t *err;
+};
+
+// the MMAs of D (TMEM) = A W^T, A [128][K], W [N][K], without the commit
+__device__ __forceinline__ void tc_product(uint32_t tmem_d, uint32_t a_base, uint32_t w_base, int K, int N) {
+  const uint32_t lbo_a = (kTcRows / 8) * 128, lbo_w = (uint32_t)(N / 8) * 128, idesc = umma_idesc(N);
+  for (int s = 0; s < K / 16; s++)
+    umma_bf16(tmem_d, umma_desc(a_base + 2 * s * lbo_a, lbo_a, 128), umma_desc(w_base + 2 * s * lbo_w, lbo_w, 128),
+              idesc, s > 0 ? 1u : 0u);
+}
+
+// [R][K] row-major weights into the chunk-major layout by cp.async
+__device__ __forceinline__ void tc_load_async(unsigned char *dst, const bf16 *src, int R, int K) {
+  for (int i = threadIdx.x; i < R * (K / 8); i += blockDim.x) {
+    const int r = i / (K / 8), c = i % (K / 8);
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + umma_off(r, 8 * c, R));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + r * K + 8 * c) : "memory");
+  }
+}
+
+// 16 columns of row m: into the row-major operand (unless rowm is null) and into the transposed one
+// [column][row], where a pair of lanes exchanges values so that each writes two rows of one column
+__device__ __forceinline__ void tr_store16(const float v[16], int c0, int m, unsigned char *rowm, unsigned char *colm) {
+  __align__(16) __nv_bfloat162 h[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+  if (rowm) {
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+      *reinterpret_cast<uint4 *>(rowm + umma_off(m, c0 + 8 * c, kTcRows)) = reinterpret_cast<const uint4 *>(h)[c];
+  }
+  const uint32_t *u = reinterpret_cast<const uint32_t *>(h);
+  const int odd = m & 1;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const uint32_t o = __shfl_xor_sync(0xffffffffu, u[j], 1);
+    const uint32_t w = odd ? __byte_perm(o, u[j], 0x7632) : __byte_perm(u[j], o, 0x5410);
+    *reinterpret_cast<uint32_t *>(colm + umma_off(c0 + 2 * j + odd, m & ~1, kTcRows)) = w;
+  }
+}
+
+// sums of 16 columns over the warp's 32 rows, in FP64 and added to out[0..16): halves of the columns
+// are exchanged between lanes step by step, so 15 + 1 shuffles do for 16 columns
+__device__ __forceinline__ void tr_colsum16(const float v[16], double *out) {
+  const int lane = threadIdx.x & 31;
+  double d[16];
+#pragma unroll
+  for (int j = 0; j < 16; j++) d[j] = (double)v[j];
+#pragma unroll
+  for (int n = 8; n >= 1; n >>= 1) {  // lanes with bit 2n set keep the upper n columns
+    const bool up = lane & (2 * n);
+#pragma unroll
+    for (int j = 0; j < n; j++) {
+      const double send = up ? d[j] : d[j + n], keep = up ? d[j + n] : d[j];
+      d[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * n);
+    }
+  }
+  d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
+  if (!(lane & 1)) atomicAdd(out + (lane >> 1), d[0]);
+}
+
+__global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(MlpTrainK p) {
+  extern __shared__ __align__(1024) unsigned char tr_smem[];
+  unsigned char *wb0 = tr_smem + kTrWB0, *wb1 = tr_smem + kTrWB1, *w4 = tr_smem + kTrW4, *w4t = tr_smem + kTrW4t,
+                *xT = tr_smem + kTrXT, *a3T = tr_smem + kTrA3T, *act = tr_smem + kTrAct;
+  float *bias = reinterpret_cast<float *>(tr_smem + kTrBias);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(tr_smem + kTrBar);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tr_smem + kTrBar + 8);
+  const int tid = threadIdx.x, m = tid & (kTcRows - 1), h = tid / kTcRows, warp = tid >> 5;
+  const int row = blockIdx.x * kTcRows + m;
+  const bool live = row < p.batch;
+  const int64_t src = live ? p.rows[row] : 0;
+
+  tc_load_async(wb0, p.wb + mlp_wboff(0), kMlpW, kMlpK1);
+  tc_load_async(wb1, p.wb + mlp_wboff(1), kMlpW, kMlpW);
+  tc_load_async(w4, p.wb + mlp_wboff(3), kMlpOutPad, kMlpW);
+  tc_load_async(w4t, p.wt + mlp_wboff(3), kMlpW, kMlpOutPad);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int c = 5 * h; c < 5 * h + 5; c++) {  // the input row, both layouts
+    const uint4 u = live ? reinterpret_cast<const uint4 *>(p.X + src * kMlpK1)[c] : make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4 *>(act + umma_off(m, 8 * c, kTcRows)) = u;
+    const bf16 *b = reinterpret_cast<const bf16 *>(&u);
+#pragma unroll
+    for (int j = 0; j < 8; j++) *reinterpret_cast<bf16 *>(xT + umma_off(8 * c + j, m, kMlpK1)) = b[j];
+  }
+  for (int i = tid; i < 3 * kMlpW + kMlpOutPad; i += kTrThreads) {
+    float v = 0.f;
+    if (i < 3 * kMlpW) v = p.master[mlp_boff(i / kMlpW) + i % kMlpW];
+    else if (i - 3 * kMlpW < kMlpOut) v = p.master[mlp_boff(3) + i - 3 * kMlpW];
+    bias[i] = v;
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[0])));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  const uint32_t bar = smem_u32(&bars[0]);
+  uint32_t phase = 0;
+  bool ok = true;
+  // all shared-memory writes (copies included) and tensor-memory reads so far before the next products
+  auto ready = [&]() {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+  };
+  auto done = [&]() {  // the products issued last are complete (false: the bounded wait gave up)
+    ok = __syncthreads_and(mbar_wait(bar, phase));
+    phase ^= 1u;
+    tc_fence_after();
+    return ok;
+  };
+  ready();
+  const uint32_t tmem = *tmem_slot, tz3 = tmem + 256, twork = tmem + 384;
+  const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
+  const uint32_t s_act = smem_u32(act), s_wb0 = smem_u32(wb0), s_wb1 = smem_u32(wb1), s_a3T = smem_u32(a3T);
+  do {
+    // ---- forward: layer l reads the weights of buffer l & 1 and frees it for the matrix needed after next
+#pragma unroll 1
+    for (int l = 0; l < 3; l++) {
+      if (l) ready();
+      if (tid == 0) {
+        tc_product(tmem + 128 * l, s_act, l & 1 ? s_wb1 : s_wb0, l ? kMlpW : kMlpK1, kMlpW);
+        umma_commit(bar);
+      }
+      if (!done()) break;
+      tc_load_async(l & 1 ? wb1 : wb0, l == 0 ? p.wb + mlp_wboff(2) : (l == 1 ? p.wt + mlp_wboff(2) : p.wt + mlp_wboff(1)),
+                    kMlpW, kMlpW);  // W3, then W3^T and W2^T for the backward pass
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      unsigned char *aT = tr_smem + kTrA1T + l * kTcAct;
+#pragma unroll 1
+      for (int c0 = 64 * h; c0 < 64 * h + 64; c0 += 16) {
+        float v[16];
+        tmem_ld16(tmem + lanes + (uint32_t)(128 * l + c0), v);
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] = gelu_f(v[j] + bias[l * kMlpW + c0 + j]);
+        tr_store16(v, c0, m, act, aT);
+      }
+    }
+    if (!ok) break;
+    ready();
+    if (tid == 0) {
+      tc_product(twork, s_act, smem_u32(w4), kMlpW, kMlpOutPad);
+      umma_commit(bar);
+    }
+    if (!done()) break;
+    // ---- loss and dY (kept in BF16 as the operand of its two products)
+    if (h == 0) {
+      float y[4], dy[16];
+      tmem_ld4(twork + lanes, y);
+      float s = 0.f;
+      const float sc = 2.0f / (3.0f * p.batch);
+#pragma unroll
+      for (int c = 0; c < 16; c++) {
+        dy[c] = 0.f;
+        if (c < kMlpOut && live) {
+          const float e = y[c] + bias[3 * kMlpW + c] - p.T[src * kMlpOut + c];
+          s += e * e;
+          dy[c] = sc * e;
+        }
+      }
+      __align__(16) __nv_bfloat162 q[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) q[j] = __floats2bfloat162_rn(dy[2 * j], dy[2 * j + 1]);
+#pragma unroll
+      for (int c = 0; c < 2; c++)
+        *reinterpret_cast<uint4 *>(act + umma_off(m, 8 * c, kTcRows)) = reinterpret_cast<const uint4 *>(q)[c];
+      const bf16 *qb = reinterpret_cast<const bf16 *>(q);
+#pragma unroll
+      for (int c = 0; c < 16; c++) *reinterpret_cast<bf16 *>(w4 + umma_off(c, m, kMlpOutPad)) = qb[c];  // dY^T
+      s = warp_sum(s);
+      if ((tid & 31) == 0) atomicAdd(p.loss, s / (3.0f * p.batch));
+      for (int c = 0; c < kMlpOut; c++) {
+        double d = (double)dy[c];
+        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if ((tid & 31) == 0) atomicAdd(p.gbias + 3 * kMlpW + c, d);
+      }
+    }
+    // ---- dW4^T = a3^T dY
+    ready();
+    if (tid == 0) {
+      tc_product(twork, s_a3T, smem_u32(w4), kTcRows, kMlpOutPad);
+      umma_commit(bar);
+    }
+    if (!done()) break;
+    if (h == 0) {
+      float v[4];
+      tmem_ld4(twork + lanes, v);
+      for (int c = 0; c < kMlpOut; c++) atomicAdd(p.grad + mlp_woff(3) + c * kMlpW + m, v[c]);
+    }
+    ready();
+    if (tid == 0) {  // da3 = dY W4
+      tc_product(twork, s_act, smem_u32(w4t), kMlpOutPad, kMlpW);
+      umma_commit(bar);
+    }
+    if (!done()) break;
+    // ---- backward: dz_l = da_l gelu'(z_l), then dW_l = dz_l^T a_(l-1) and da_(l-1) = dz_l W_l
+#pragma unroll 1
+    for (int l = 2; l >= 0; l--) {
+#pragma unroll 1
+      for (int c0 = 64 * h; c0 < 64 * h + 64; c0 += 16) {
+        float v[16], z[16];
+        tmem_ld16(twork + lanes + (uint32_t)c0, v);
+        tmem_ld16(tmem + lanes + (uint32_t)(128 * l + c0), z);
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] *= gelu_grad_f(z[j] + bias[l * kMlpW + c0 + j]);
+        tr_store16(v, c0, m, l ? act : nullptr, a3T);
+        tr_colsum16(v, p.gbias + l * kMlpW + c0);
+      }
+      ready();
+      const int K = l ? kMlpW : kMlpK1;  // inputs of the layer
+      if (tid == 0) {
+        tc_product(tz3, s_a3T, smem_u32(l ? tr_smem + kTrA1T + (l - 1) * kTcAct : xT), kTcRows, K);
+        if (l) tc_product(twork, s_act, l == 2 ? s_wb1 : s_wb0, kMlpW, kMlpW);
+        umma_commit(bar);
+      }
+      if (!done()) break;
+      float *g = p.grad + mlp_woff(l) + m * K;
+      const int cb = l ? 64 : 48;  // first column of the upper half
+#pragma unroll 1
+      for (int c0 = h ? cb : 0; c0 < (h ? K : cb); c0 += 16) {
+        float v[16];
+        tmem_ld16(tz3 + lanes + (uint32_t)c0, v);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          atomicAdd(reinterpret_cast<float4 *>(g + c0) + j, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+      }
+    }
+  } while (false);
+  if (!ok) {
+    // a wait gave up while products may still run: wait once more (also bounded) before the tensor memory goes
+    if (tid == 0) atomicOr(p.err, 1 << CUBE_ERR_TIMEOUT);
+    (void)mbar_wait(bar, phase ^ 1u);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  }
+}
+
+// Adam on the FP32 master parameters (bias gradients arrive in FP64), and the BF16 weight copies
+__global__ void k_adam_pack(float *w, float *grad, const double *gbias, float *m, float *v, bf16 *wb, bf16 *wt, float lr,
+                            float b1, float b2, float eps, float c1, float c2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kMlpParams) return;
+  int l = 0;
+  while (l < 3 && i >= mlp_woff(l + 1)) l++;
+  const int e = i - mlp_woff(l), K = mlp_K(l);
+  const bool isb = i >= mlp_boff(l);
+  float gi = grad[i];
+  if (isb) grad[i] = gi = (float)gbias[l * kMlpW + i - mlp_boff(l)];
+  const float mi = b1 * m[i] + (1.f - b1) * gi, vi = b2 * v[i] + (1.f - b2) * gi * gi;
+  m[i] = mi;
+  v[i] = vi;
+  const float x = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  w[i] = x;
+  if (!isb) {
+    const bf16 b = __float2bfloat16_rn(x);
+    const int n = e / K, k = e - n * K;
+    wb[mlp_wboff(l) + e] = b;
+    wt[mlp_wboff(l) + k * mlp_Np(l) + n] = b;
   }
 }
 
@@ -969,9 +1262,9 @@ void launch_mlp_features(const float4 *pos, int64_t n, const float *rho, int ng,
   k_mlp_features<<<148 * 8, 256, 0, s>>>(pos, n, rho, ng, X);
 }
 
-// The training GEMMs run on tcgen05 (k_gemm_nt_tc); CUBE_MLP_MMA_SYNC selects the mma.sync
+// The forward GEMMs run on tcgen05 (k_gemm_nt_tc); CUBE_MLP_MMA_SYNC selects the mma.sync
 // kernel instead (kept as an independent cross-check).
-static int32_t *g_gemm_err = nullptr;  // status word of the current training call (MlpParams::err)
+static int32_t *g_gemm_err = nullptr;  // status word of the current call (MlpParams::err)
 
 void launch_gemm_nt(const bf16 *A, int lda, const bf16 *B, int ldb, int M, int N, int K, const float *bias, float *Z,
                     int ldz, bf16 *H, int ldh, int act, cudaStream_t s) {
@@ -983,11 +1276,7 @@ void launch_gemm_nt(const bf16 *A, int lda, const bf16 *B, int ldb, int M, int N
       cudaFuncSetAttribute(k_gemm_nt_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGtSmem);
       attr_dev = dev;
     }
-    // long K (the weight gradients sum over the batch) on few output tiles: split K over CTAs
-    int split = 1;
-    if (Z && !H && !bias && !act && M <= 2 * kGtM && K >= 4 * kGtK) split = std::min(32, K / (4 * kGtK));
-    if (split > 1) cudaMemset2DAsync(Z, sizeof(float) * (size_t)ldz, 0, sizeof(float) * (size_t)N, (size_t)M, s);
-    dim3 grid((unsigned)((N + kGtN - 1) / kGtN), (unsigned)((M + kGtM - 1) / kGtM), (unsigned)split);
+    dim3 grid((unsigned)((N + kGtN - 1) / kGtN), (unsigned)((M + kGtM - 1) / kGtM));
     k_gemm_nt_tc<<<grid, kGtM, kGtSmem, s>>>(A, lda, B, ldb, M, N, K, bias, Z, ldz, H, ldh, act, g_gemm_err);
     return;
   }
@@ -1011,10 +1300,10 @@ void launch_mlp_apply(const MlpParams &m, const float4 *pos, const float *rho, i
   }
 }
 
-// Forward + backward + Adam on one batch of `batch` rows picked by `rows` from X / T.
-int mlp_train_step(MlpParams &m, const bf16 *X, const float *T, const int32_t *rows, int batch, float lr,
-                   float *loss, cudaStream_t s) {
-  if (batch <= 0 || batch > m.cap || batch % 16) return CUBE_ERR_INVALID;
+// The same step as separate GEMMs, transposes and elementwise passes on mma.sync: an independent
+// cross-check of k_mlp_train, run when CUBE_MLP_MMA_SYNC is set.
+static int train_step_separate(MlpParams &m, const bf16 *X, const float *T, const int32_t *rows, int batch, float lr,
+                               float *loss, cudaStream_t s) {
   g_gemm_err = m.err;
   const int B = batch, W = kMlpW, OP = kMlpOutPad;
   const int g1 = 148 * 8;
@@ -1059,7 +1348,31 @@ int mlp_train_step(MlpParams &m, const bf16 *X, const float *T, const int32_t *r
   return cudaGetLastError() == cudaSuccess ? CUBE_OK : CUBE_ERR_CUDA;
 }
 
-// Y[rows][3] of X through the training GEMM path (no kick): for checks against the oracle
+// Forward + backward + Adam on one batch of `batch` rows picked by `rows` from X / T.
+int mlp_train_step(MlpParams &m, const bf16 *X, const float *T, const int32_t *rows, int batch, float lr,
+                   float *loss, cudaStream_t s) {
+  if (batch <= 0 || batch > m.cap || batch % 16) return CUBE_ERR_INVALID;
+  if (getenv("CUBE_MLP_MMA_SYNC")) return train_step_separate(m, X, T, rows, batch, lr, loss, s);
+  static int attr_dev = -1;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (attr_dev != dev) {
+    cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrSmem);
+    attr_dev = dev;
+  }
+  double *gbias = reinterpret_cast<double *>(m.grad + kMlpGradBias);
+  cudaMemsetAsync(m.grad, 0, kMlpGradBytes, s);
+  MlpTrainK p{X, T, rows, batch, m.wb, m.wt, m.master, m.grad, gbias, loss, m.err};
+  k_mlp_train<<<(batch + kTcRows - 1) / kTcRows, kTrThreads, kTrSmem, s>>>(p);
+  m.step += 1;
+  const float b1 = 0.9f, b2 = 0.999f;
+  const float c1 = 1.f - powf(b1, (float)m.step), c2 = 1.f - powf(b2, (float)m.step);
+  k_adam_pack<<<(kMlpParams + 255) / 256, 256, 0, s>>>(m.master, m.grad, gbias, m.mom, m.vel, m.wb, m.wt, lr, b1, b2,
+                                                      1e-8f, c1, c2);
+  return cudaGetLastError() == cudaSuccess ? CUBE_OK : CUBE_ERR_CUDA;
+}
+
+// Y[rows][3] of X layer by layer (no kick): for checks against the oracle
 int mlp_forward(MlpParams &m, const bf16 *X, int64_t nrows, float *Y, cudaStream_t s) {
   g_gemm_err = m.err;
   const int W = kMlpW, OP = kMlpOutPad;
