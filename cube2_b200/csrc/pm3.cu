@@ -437,54 +437,6 @@ __device__ __forceinline__ BrickPos brick_pos(const PM3K &p, int64_t b, int cb, 
   return q;
 }
 
-// ---- mbarrier and bulk-copy helpers (sm_90+) ----
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-// arrive on the mbarrier and expect `bytes` of asynchronous copies in the same phase
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(
-                   smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred P1;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, P1;\n\t}\n"
-      : "=r"(done)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-__device__ __forceinline__ unsigned long long ns_now() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-constexpr unsigned long long kBulkWaitNs = 1000000000ull;  // bound of one wait for a brick's copies: 1 s
-// wait for a phase of the mbarrier, at most kBulkWaitNs; false when the wait gave up
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity) {
-  const unsigned long long t0 = ns_now();
-  while (!mbar_try_wait(bar, parity))
-    if (ns_now() - t0 > kBulkWaitNs) return false;
-  return true;
-}
-// bulk asynchronous copy global -> this CTA's shared memory, completing on the mbarrier
-// (both addresses 16-byte aligned, bytes a multiple of 16)
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
-
 // Force and gather in one pass, persistent and warp-specialised: one 1024-thread block per SM
 // claims bricks from a work counter.  Its producer warps (the first kFgProd threads) compute a
 // brick's force window while its consumer warps gather the previous brick, so the two phases

@@ -13,28 +13,21 @@
 // heaviest first through an atomic queue head, so the lognormal occupancy of
 // clustered boxes does not leave a tail.
 //
-// Inside an item one warp splits its 32 lanes into floor(32/ni) groups of ni
-// lanes; lane (group g, particle i) walks every ngrp-th staged candidate.  The
-// needed rows are laid end to end in a per-warp row table, so every staging
-// step loads 32 candidates (prefetched one step ahead) however short the rows
-// are.  A candidate is staged in shared memory only if it lies within rc of
-// the bounding box of the item's particles, which removes most of the stencil
-// volume before the pair law runs.  The pair law is evaluated without
-// divisions or selects: the inner piece of the S2 law differs from the outer
-// one by (1 - ep)^6 (12 + 72 ep + 28 ep^2) / ep^2, so one Horner polynomial in
-// r plus max(1 - ep, 0)^6 times a quadratic covers both.  Each lane keeps
-// Kahan-compensated sums updated once per flush of the staging buffer; the
-// groups of a particle are merged with warp shuffles (TwoSum), and the owning
-// lane applies af*mass^2, the kick, f2max and vmax.
+// The kick runs k_pp_pairs: per item, the stencil's rows arrive in shared memory by bulk copies, candidates
+// beyond rc of the bounding box of the item's particles are dropped, a TF32 tensor-core product
+// lists for every particle the candidates that can lie within rc, and only the listed pairs are
+// evaluated, in FP32 on f32x2 arithmetic (FFMA2, FMUL2, FADD2: two pairs per lane and
+// instruction; every operation rounds as its scalar form).  Sums are Kahan-compensated over the
+// batches of an item and merged with TwoSum shuffles, and the owning lane applies af*mass^2, the
+// kick, f2max and vmax.
 //
-// Packed shapes evaluate the pair law on sm_100's f32x2 arithmetic (FFMA2, FMUL2, FADD2):
-// a lane takes two staged candidates per round, which halves the issue slots of the law;
-// every operation rounds as its scalar form, so each pair's force is bit for bit the scalar
-// one and only the summation order differs.  The kernel is issue-bound, so the per-lane state
-// that is touched once per flush or item (Kahan sums, maxima, the owned particle's velocity,
-// which a cp.async brings in while the item runs) lives in shared memory, and a warp pops
-// its work items four at a time, each carrying its first particle, count, stencil radius
-// and pair-law constants (k_pp_items computes them once per kick).
+// k_pp_force is the scalar form (the pair count and the comparison shapes): lane (group g,
+// particle i) of floor(32/ni) groups evaluates every ngrp-th candidate that passes the box test.
+//
+// Both kernels are issue-bound, so the per-lane state that is touched once per batch or item (Kahan sums,
+// maxima, the owned particle's velocity, which a cp.async brings in while the item runs) lives in
+// shared memory, and a warp pops its work items up to four at a time, each carrying its first
+// particle, count, stencil radius and pair-law constants (k_pp_items computes them once per kick).
 #include <type_traits>
 #include <utility>
 
@@ -44,20 +37,20 @@ namespace cube {
 
 constexpr int kPPThreads = 256;
 constexpr int kPPWarps = kPPThreads / 32;
-constexpr int kMaxRows = 96;  // stencil rows per row table (a multiple of 32)
+constexpr int kMaxRows = 96;  // stencil rows per row table of the scalar kernel (a multiple of 32)
 constexpr int kBuckets = 32;
+constexpr float kFar = 1e7f;  // coordinate of a padding candidate: beyond every range, and its law stays finite
 
 // Kernel shapes the autotuner picks from (the host times each on the kick's own particles):
 // chunk = i-particles per work item, so a crowded PP cell of n particles gets ceil(n / chunk)
 // warps; jtile = candidates a warp stages in shared memory between two flushes; unroll = unroll
-// factor of the pair loop; blocks = resident blocks per SM the registers are budgeted for
-// (4: 64 registers a thread, 3: 80), packed = pair law on f32x2 arithmetic.  Shape 0 is the
-// default; the last shape is the scalar form, kept for comparison.
+// factor of the filter loop (packed) or the pair loop (scalar); blocks = resident blocks per SM
+// the registers are budgeted for (4: 64 registers a thread, 3: 80), packed = the pair-list kernel
+// k_pp_pairs with the law on f32x2 arithmetic.  Shape 0 is the default; the scalar shapes
+// (k_pp_force) are kept for comparison.
 constexpr PPShapeDesc kShapes[] = {
-    {16, 128, 2, 4, 1}, {16, 128, 1, 4, 1}, {16, 256, 2, 4, 1}, {16, 128, 4, 4, 1}, {16, 64, 2, 4, 1},
-    {16, 128, 2, 3, 1}, {16, 256, 1, 4, 1}, {8, 256, 1, 4, 1},  {8, 256, 2, 4, 1},  {16, 128, 8, 4, 1},
-    {32, 128, 2, 4, 1}, {16, 256, 4, 4, 1}, {16, 96, 4, 4, 1},  {16, 64, 4, 4, 1},  {16, 64, 1, 4, 1},
-    {16, 64, 2, 4, 0}};
+    {16, 224, 4, 4, 1}, {16, 256, 4, 4, 1}, {16, 224, 2, 4, 1}, {16, 128, 4, 4, 1}, {16, 256, 4, 3, 1},
+    {8, 224, 4, 4, 1},  {8, 128, 4, 4, 1},  {16, 64, 2, 4, 0},  {32, 64, 2, 4, 0}};
 // the pair-count kernel (scalar loop, the work list of shape 0)
 constexpr PPShapeDesc kCountShape = {kShapes[0].chunk, 64, 2, 4, 0};
 constexpr int kNumShapes = (int)(sizeof(kShapes) / sizeof(kShapes[0]));
@@ -69,28 +62,23 @@ constexpr int min_shape_chunk() {
 }
 constexpr int kMinChunk = min_shape_chunk();  // the work list capacity is sized for it
 static_assert(kShapes[0].chunk == kPPChunk, "shape 0 is the default shape");
-// per-warp shared memory: the staged candidates (scalar: float4 [jtile + 32]; packed: x, y and z
-// planes of jtile + 64 floats each), then the row table
-constexpr size_t pp_stage_bytes(int jtile, bool packed) {
-  return packed ? 3 * sizeof(float) * (jtile + 64) : sizeof(float4) * (jtile + 32);
+// Per-warp shared memory: the staged candidates (float4 [jtile + 32]), then the per-lane state kept in
+// shared memory rather than registers (it is touched once per flush or item): f2 and |v| maxima, the
+// owned particle's velocity (copied in asynchronously while the item runs), Kahan sums and
+// compensations; then the batch of work items the warp popped, and the mbarrier of its copies.  The
+// scalar kernel adds its row table, the item's bounding box and the row-table cache.
+constexpr int kLaneFieldsScalar = 13, kLaneFieldsPairs = 19;
+constexpr int kPop = 4;  // most work items a warp takes from the queue at a time
+constexpr int kRefill = 96;  // pair kernel: a batch of candidates is evaluated once less room than this is left
+constexpr size_t pp_stage_bytes(int jtile) { return sizeof(float4) * (jtile + 32); }
+constexpr size_t pp_smem_warp(int jtile, bool pairs) {
+  return pp_stage_bytes(jtile) + sizeof(PPItem) * kPop +
+         (pairs ? sizeof(float) * 32 * kLaneFieldsPairs + 16
+                : sizeof(float) * (32 * kLaneFieldsScalar + 8) + sizeof(int2) * kMaxRows);
 }
-// per-lane state kept in shared memory rather than registers (it is touched once per flush or
-// item): Kahan sums and compensations of x, y, z, f2 and |v| maxima, the owned particle's
-// velocity (copied in asynchronously when the item starts); then the item's bounding box and
-// the row-table cache, then the batch of work items the warp popped
-constexpr int kLaneFields = 13;
-constexpr int kPop = 4;  // work items a warp takes from the queue at a time
-constexpr size_t pp_state_bytes() { return sizeof(float) * (kLaneFields * 32 + 8) + sizeof(PPItem) * kPop; }
-constexpr size_t pp_smem_warp(int jtile, bool packed) {
-  return pp_stage_bytes(jtile, packed) + sizeof(int2) * kMaxRows + pp_state_bytes();
-}
-constexpr size_t pp_smem_block(int jtile, bool packed) { return pp_smem_warp(jtile, packed) * kPPWarps; }
-constexpr bool pp_smem_aligned() {
-  for (int jt = 32; jt <= 256; jt += 32)
-    if (pp_smem_warp(jt, false) % 16 || pp_smem_warp(jt, true) % 16 || pp_stage_bytes(jt, true) % 16) return false;
-  return true;
-}
-static_assert(pp_smem_aligned() && (sizeof(int2) * kMaxRows + sizeof(float) * 32 * kLaneFields) % 16 == 0,
+constexpr size_t pp_smem_block(int jtile, bool pairs) { return pp_smem_warp(jtile, pairs) * kPPWarps; }
+static_assert(pp_smem_warp(64, false) % 16 == 0 && pp_smem_warp(224, true) % 16 == 0 &&
+                  (sizeof(int2) * kMaxRows) % 16 == 0,
               "16-byte aligned warp areas, bounding box and item batch");
 
 // F_ra(r, apm) of basic_functions.f08:95-109 / pp_force_kernel.c:45-74 in FP32 without
@@ -132,16 +120,19 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// s(r^2) = (F_ra(r,app) - F_ra(r,rc)) / r for 0 <= r < rc, so that the pair force is s * (dx, dy, dz).
-// With ep = 2r/rc and k = 1/(35 rc^2), for r > app:
-//   outer (ep > 1): 1/r^2 - F_ra(r,rc) = (32/35)/r^2 - k P(ep),  P = -224 + 896ep - 840ep^2 + 224ep^3
-//                                                                     + 70ep^4 - 48ep^5 + 7ep^6
-//   inner (ep <= 1): the outer form plus k (1-ep)^6 (12 + 72ep + 28ep^2) / ep^2
-//                    = (1/r^2) (1-ep)^6 (3/35 + 18/35 ep + 7/35 ep^2)
-// (expanding the product gives back the inner polynomial 224ep - 224ep^3 + 70ep^4 + 48ep^5 - 21ep^6).
-// The polynomial coefficients are literals (instruction immediates), so a law costs two registers
-// per item (2/rc and 1/(35 rc^2)).  Inside the softening length (soft(), a second pass over
-// the pairs the main loop flags) both F_ra terms are evaluated directly.
+// s(r^2) = (F_ra(r,app) - F_ra(r,rc)) / r, so that the pair force is s * (dx, dy, dz).  With
+// ep = 2r/rc and k = 1/(35 rc^2), for app < r:
+//   outer (1 < ep < 2): 1/r^2 - F_ra(r,rc) = k/ep^2 (128 + 224ep^2 - 896ep^3 + 840ep^4 - 224ep^5 - 70ep^6
+//                       + 48ep^7 - 7ep^8) = k/ep^2 (2-ep)^5 (4 + 10ep + 22ep^2 + 7ep^3)
+//   inner (ep <= 1): the outer form plus k/ep^2 (1-ep)^6 (12 + 72ep + 28ep^2)
+// (the octic has a fivefold root at ep = 2, the difference of the two pieces a sixfold root at ep = 1), and
+// k/ep^2 / r = (1/140) / r^3.  With h = r/rc = ep/2:
+//   s = r^-3 [ (1-h)^5 (32/140) (4 + 20h + 88h^2 + 56h^3) + max(1-2h, 0)^6 (1/140) (12 + 144h + 112h^2) ].
+// Every term is positive, so the law keeps its relative accuracy up to r = rc (the expanded octic
+// cancels there: terms of 100 leave an absolute error of 6e-6); both factors lie in [0, 1], so the
+// saturating FMA gives them without a compare, and 1-h saturated makes the law exactly zero beyond rc.
+// The coefficients are literals, so a law costs one register per item (1/rc).  Inside the softening
+// length (soft()) both F_ra terms are evaluated directly.
 struct PairLaw {
   float cep, k35;
   // the constants of range rc, as k_pp_items stores them in the work item
@@ -153,40 +144,28 @@ struct PairLaw {
   }
   __device__ __forceinline__ float scale(float r2) const {
     const float invr = rsqrt_ftz(r2);
-    const float ir2 = invr * invr;
-    const float ep = r2 * invr * cep;
-    float q = fmaf(7.0f, ep, -48.0f);
-    q = fmaf(q, ep, 70.0f);
-    q = fmaf(q, ep, 224.0f);
-    q = fmaf(q, ep, -840.0f);
-    q = fmaf(q, ep, 896.0f);
-    q = fmaf(q, ep, -224.0f);
-    const float u = fmaxf(1.0f - ep, 0.0f);
-    const float u2 = u * u;
-    const float u6 = u2 * u2 * u2;
-    const float w = fmaf(fmaf(7.0f / 35.0f, ep, 18.0f / 35.0f), ep, 3.0f / 35.0f);
-    const float br = fmaf(u6, w, 32.0f / 35.0f);
-    return fmaf(br, ir2, -q * k35) * invr;
+    const float h = r2 * invr * (0.5f * cep);
+    const float v = __saturatef(1.0f - h), u = __saturatef(fmaf(-2.0f, h, 1.0f));
+    const float c = fmaf(fmaf(fmaf(1792.0f / 140.0f, h, 2816.0f / 140.0f), h, 640.0f / 140.0f), h, 128.0f / 140.0f);
+    const float w = fmaf(fmaf(112.0f / 140.0f, h, 144.0f / 140.0f), h, 12.0f / 140.0f);
+    const float v2 = v * v, u2 = u * u, u3 = u2 * u;
+    const float a = (v2 * v2) * (v * c);
+    return fmaf(u3 * u3, w, a) * (invr * invr * invr);
   }
   // scale() of two squared distances on packed f32x2 arithmetic: every operation is the scalar
   // one, rounded the same way, so each half equals scale() of that half bit for bit
   __device__ __forceinline__ float2 scale2(float2 r2) const {
     const float2 invr = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
-    const float2 ir2 = mul2(invr, invr);
-    const float2 ep = mul2(mul2(r2, invr), dup(cep));
-    float2 q = fma2(dup(7.0f), ep, dup(-48.0f));
-    q = fma2(q, ep, dup(70.0f));
-    q = fma2(q, ep, dup(224.0f));
-    q = fma2(q, ep, dup(-840.0f));
-    q = fma2(q, ep, dup(896.0f));
-    q = fma2(q, ep, dup(-224.0f));
-    float2 u = fma2(ep, dup(-1.0f), dup(1.0f));
-    u = make_float2(fmaxf(u.x, 0.0f), fmaxf(u.y, 0.0f));
-    const float2 u2 = mul2(u, u);
-    const float2 u6 = mul2(mul2(u2, u2), u2);
-    const float2 w = fma2(fma2(dup(7.0f / 35.0f), ep, dup(18.0f / 35.0f)), ep, dup(3.0f / 35.0f));
-    const float2 br = fma2(u6, w, dup(32.0f / 35.0f));
-    return mul2(fma2(br, ir2, mul2(q, dup(-k35))), invr);
+    const float2 h = mul2(mul2(r2, invr), dup(0.5f * cep));
+    const float2 v = make_float2(__saturatef(1.0f - h.x), __saturatef(1.0f - h.y)),
+                 u = make_float2(__saturatef(fmaf(-2.0f, h.x, 1.0f)), __saturatef(fmaf(-2.0f, h.y, 1.0f)));
+    float2 c = fma2(dup(1792.0f / 140.0f), h, dup(2816.0f / 140.0f));
+    c = fma2(c, h, dup(640.0f / 140.0f));
+    c = fma2(c, h, dup(128.0f / 140.0f));
+    const float2 w = fma2(fma2(dup(112.0f / 140.0f), h, dup(144.0f / 140.0f)), h, dup(12.0f / 140.0f));
+    const float2 v2 = mul2(v, v), u2 = mul2(u, u), u3 = mul2(u2, u);
+    const float2 a = mul2(mul2(v2, v2), mul2(v, c));
+    return mul2(fma2(mul2(u3, u3), w, a), mul2(mul2(invr, invr), invr));
   }
   // 0 < r <= app: (F_ra(r, app) - F_ra(r, rc)) / r; cea = 2/app, ka = (1/35)/app^2
   __device__ __forceinline__ float soft(float r2, float cea, float ka) const {
@@ -196,17 +175,16 @@ struct PairLaw {
   }
 };
 
-// order-preserving map between floats and ints, for the integer warp reductions (redux.sync)
-__device__ __forceinline__ int float_key(float f) {
-  const int i = __float_as_int(f);
-  return i >= 0 ? i : i ^ 0x7fffffff;
-}
-__device__ __forceinline__ float key_float(int k) { return __int_as_float(k >= 0 ? k : k ^ 0x7fffffff); }
+// warp minimum / maximum of a float in one instruction (sm_100a)
 __device__ __forceinline__ float warp_min_redux(float v) {
-  return key_float(__reduce_min_sync(0xffffffffu, float_key(v)));
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
 __device__ __forceinline__ float warp_max_redux(float v) {
-  return key_float(__reduce_max_sync(0xffffffffu, float_key(v)));
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
 
 // n / d for 0 <= n < 2^11 and 1 <= d <= 64 by a multiply with ceil(2^20 / d): the error
@@ -460,26 +438,22 @@ __global__ void k_pp_offsets(int32_t *sched, int ntile) {
 // COUNT = false: forces and kick.  COUNT = true: only count the accepted ordered
 // pairs 0 < r^2 < rc^2 (the algorithmic work of the kick, for the roofline).
 // Shape: C i-particles per item, J staged candidates per flush, pair loop unrolled U times,
-// registers budgeted for B resident blocks per SM, pair law on packed f32x2 arithmetic (PK).
-template <bool COUNT, int C, int J, int U, int B, bool PK>
+// registers budgeted for B resident blocks per SM.
+template <bool COUNT, int C, int J, int U, int B>
 __global__ void __launch_bounds__(kPPThreads, B) k_pp_force(PPK p) {
-  // a flush has at most ceil(J / floor(32 / C)) rounds (packed: pair rounds, two candidates
-  // each), one bit per round and lane in the soft-pair mask
-  constexpr int kNg = 32 / C;
-  constexpr int kBits = PK ? (J + 2 * kNg - 1) / (2 * kNg) : (J + kNg - 1) / kNg;
+  // a flush has at most ceil(J / floor(32 / C)) rounds, one bit per round and lane in the
+  // soft-pair mask
+  constexpr int kBits = (J + 32 / C - 1) / (32 / C);
   static_assert(kBits <= 64, "at most 64 soft-pair bits per flush");
-  static_assert(!(COUNT && PK), "the pair count runs the scalar loop");
   using Mask = typename std::conditional<(kBits > 32), unsigned long long, unsigned>::type;
   extern __shared__ float4 pp_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  char *wbase = reinterpret_cast<char *>(pp_smem) + warp * pp_smem_warp(J, PK);
-  float4 *buf = reinterpret_cast<float4 *>(wbase);  // scalar staging: float4 [J + 32]
-  float *X = reinterpret_cast<float *>(wbase);      // packed staging: planes of J + 64 floats
-  float *Y = X + (J + 64), *Z = Y + (J + 64);
+  char *wbase = reinterpret_cast<char *>(pp_smem) + warp * pp_smem_warp(J, false);
+  float4 *buf = reinterpret_cast<float4 *>(wbase);  // staging: float4 [J + 32]
   // (end of the row in the walk, start - walk offset)
-  int2 *rows = reinterpret_cast<int2 *>(wbase + pp_stage_bytes(J, PK));
+  int2 *rows = reinterpret_cast<int2 *>(wbase + pp_stage_bytes(J));
   float *const ks = reinterpret_cast<float *>(rows + kMaxRows) + lane;  // field f at ks[32 f]
-  float *const bbox = reinterpret_cast<float *>(rows + kMaxRows) + 32 * kLaneFields;
+  float *const bbox = reinterpret_cast<float *>(rows + kMaxRows) + 32 * kLaneFieldsScalar;
   PPItem *const batch = reinterpret_cast<PPItem *>(bbox + 8);
   int *const tcache = reinterpret_cast<int *>(bbox + 6);  // cell and walk of the row table
   if (lane == 0) tcache[0] = -1;
@@ -526,67 +500,8 @@ __global__ void __launch_bounds__(kPPThreads, B) k_pp_force(PPK p) {
     // no branch: pairs inside the softening length (r <= app, common only in dense clumps) are
     // masked out of it and their rounds recorded in a bit mask (at most 32 rounds per flush);
     // a second loop then evaluates exactly those pairs, one per lane per step.
-    // Packed: candidates 2m and 2m + 1 form pair slot m, and group grp takes slots grp + k*ngrp;
-    // its two halves are summed separately and added at the end of the flush.
-    auto flush_packed = [&]() {
-      X[nbuf + lane] = 1e18f;
-      Y[nbuf + lane] = 1e18f;
-      Z[nbuf + lane] = 1e18f;
-      X[nbuf + 32 + lane] = 1e18f;
-      Y[nbuf + 32 + lane] = 1e18f;
-      Z[nbuf + 32 + lane] = 1e18f;
-      __syncwarp();
-      float2 px = dup(0.f), py = dup(0.f), pz = dup(0.f);
-      const int nround = div_small(nbuf + 2 * ngrp - 1, 2 * ngrp);
-      Mask softmask = 0u, bit = 1u;
-      const float2 *X2 = reinterpret_cast<const float2 *>(X);
-      const float2 nx = dup(-pi.x), ny = dup(-pi.y), nz = dup(-pi.z);
-      int m = grp;
-#pragma unroll U
-      for (int k = 0; k < nround; k++, m += ngrp, bit <<= 1) {
-        const float2 dx = add2(X2[m], nx), dy_ = add2(X2[m + (J + 64) / 2], ny),
-                     dz_ = add2(X2[m + (J + 64)], nz);
-        const float2 r2 = fma2(dx, dx, fma2(dy_, dy_, mul2(dz_, dz_)));
-        float2 s = law.scale2(r2);
-        const bool fx = r2.x > p.app2, fy = r2.y > p.app2;
-        s.x = fx & (r2.x < rc2) ? s.x : 0.0f;
-        s.y = fy & (r2.y < rc2) ? s.y : 0.0f;
-        if ((!fx & (r2.x > 0.0f)) | (!fy & (r2.y > 0.0f))) softmask |= bit;
-        px = fma2(s, dx, px);
-        py = fma2(s, dy_, py);
-        pz = fma2(s, dz_, pz);
-      }
-      if (!has_i) softmask = 0u;
-      // a flagged pair round holds one or two soft pairs: both halves are tested again
-      while (__any_sync(0xffffffffu, softmask != 0u)) {
-        if (softmask) {
-          const int c = 2 * (grp + lowest_bit(softmask) * ngrp);
-          softmask &= softmask - 1u;
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const float dx = X[c + e] - pi.x, dy_ = Y[c + e] - pi.y, dz_ = Z[c + e] - pi.z;
-            const float r2 = fmaf(dx, dx, fmaf(dy_, dy_, dz_ * dz_));
-            if ((r2 <= p.app2) & (r2 > 0.0f)) {
-              const float s = law.soft(r2, p.cea, p.ka);
-              px.x = fmaf(s, dx, px.x);
-              py.x = fmaf(s, dy_, py.x);
-              pz.x = fmaf(s, dz_, pz.x);
-            }
-          }
-        }
-      }
-      kahan_add(ks[0], ks[32], px.x + px.y);
-      kahan_add(ks[64], ks[96], py.x + py.y);
-      kahan_add(ks[128], ks[160], pz.x + pz.y);
-      nbuf = 0;
-      __syncwarp();
-    };
     auto flush = [&]() {
-      if constexpr (PK) {
-        flush_packed();
-        return;
-      }
-      buf[nbuf + lane] = make_float4(1e18f, 1e18f, 1e18f, 0.f);
+      buf[nbuf + lane] = make_float4(kFar, kFar, kFar, 0.f);
       __syncwarp();
       float px = 0.f, py = 0.f, pz = 0.f;
       const int nround = div_small(nbuf + ngrp - 1, ngrp);
@@ -716,13 +631,7 @@ __global__ void __launch_bounds__(kPPThreads, B) k_pp_force(PPK p) {
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (keep) {
           const int q = nbuf + __popc(m & ((1u << lane) - 1u));
-          if constexpr (PK) {
-            X[q] = pj.x;
-            Y[q] = pj.y;
-            Z[q] = pj.z;
-          } else {
-            buf[q] = pj;
-          }
+          buf[q] = pj;
         }
         nbuf += __popc(m);
         if (nbuf > J - 32) flush();
@@ -768,6 +677,382 @@ __global__ void __launch_bounds__(kPPThreads, B) k_pp_force(PPK p) {
   if (lane == 0) atomic_max_nonneg(&p.out[1], f2w);
   if (p.want_vmax) {
     const float vm0 = warp_max(ks[224]), vm1 = warp_max(ks[256]), vm2 = warp_max(ks[288]);
+    if (lane == 0) {
+      atomic_max_nonneg(&p.out[2], vm0);
+      atomic_max_nonneg(&p.out[3], vm1);
+      atomic_max_nonneg(&p.out[4], vm2);
+    }
+  }
+}
+
+// ---- the pair-list kernel ----
+//
+// One warp per work item, in three phases per batch of up to J candidates:
+//   stage: one bulk copy per stencil row brings its particles to shared memory; those beyond rc of the
+//     item's box are dropped in place.  (Walking the rows with one load per lane and step cost
+//     about 120 instructions per 32 candidates in finding each lane's row; this costs 40.)
+//   filter: the squared distances of the item's 16 rows (its i-particles, replicated when there are
+//     fewer than 9) to 8 candidates come from one TF32 tensor-core product (mma.m16n8k8, the
+//     contraction  -2 xi . xj + |xj|^2 + (|xi|^2 - T)  over positions relative to the box
+//     centre); the sign of each result goes into a bit list of its lane.  T is rc^2 plus the largest
+//     error that TF32 operands can make in the item's box, so no pair within rc is missed.
+//   pairs: each lane takes the candidates of its two rows' lists one after the other (two rows = the two
+//     halves of f32x2 arithmetic) and evaluates the law in FP32 from the exact positions; the few listed
+//     pairs beyond rc get exactly zero from it.
+// Lane (g, t) = (lane / 4, lane % 4) owns rows g and g + 8 against every fourth candidate (the layout of the
+// accumulator fragment; neighbouring candidates go to different lanes, which keeps the four lists of a
+// row alike in length: contiguous quarters needed 1.6 times the rounds).
+//
+// What it does instead of the law on every candidate: only one in 3 (clustered) to 5 (uniform) of the
+// pairs that pass the box test is within rc, and evaluating them all took 29 (uniform) and 39 (clustered)
+// rounds of 64 per item, against 11 and 21 rounds of the listed ones (75 instructions each, 2300
+// instead of 2950 and 3180 instead of 3610 instructions per item together with the staging).
+// It issues on 82 % of the cycles; the lists of a batch differ in length, which idles a third of the
+// pair slots.  192^3 boxes under ncu, before and after: uniform 1.67 to 1.18 ms, lognormal
+// (sigma 1.5) 3.09 to 3.00 ms with 224 candidates a batch and 4 blocks per SM, 2.9 ms with 256 and 3.
+__device__ __forceinline__ unsigned tf32_floor(float x) { return __float_as_uint(x) & 0xffffe000u; }
+__device__ __forceinline__ unsigned tf32_rna(float x) {
+  unsigned r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void mma_tf32(float d[4], const unsigned a[4], unsigned b0, unsigned b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// index of the highest set bit (-1: none), and 1 << b (0 for b = -1)
+__device__ __forceinline__ int high_bit(unsigned m) {
+  int b;
+  asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(m));
+  return b;
+}
+__device__ __forceinline__ unsigned bit_at(int b) {
+  unsigned r;
+  asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(b));
+  return r;
+}
+__device__ __forceinline__ float4 lds128(unsigned a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float lds32(unsigned a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+
+template <int C, int J, int U, int B>
+__global__ void __launch_bounds__(kPPThreads, B) k_pp_pairs(PPK p) {
+  static_assert(C <= 16 && J % 32 == 0 && J <= 256, "16 rows, two 32-bit lists a row and lane");
+  extern __shared__ float4 pp_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  char *wbase = reinterpret_cast<char *>(pp_smem) + warp * pp_smem_warp(J, true);
+  // staged candidates, relative to the box centre: x, y, z, |x|^2
+  float4 *const buf = reinterpret_cast<float4 *>(wbase);
+  const unsigned buf_s = (unsigned)__cvta_generic_to_shared(buf);
+  float *const ks = reinterpret_cast<float *>(wbase + pp_stage_bytes(J)) + lane;  // field f at ks[32 f]
+  PPItem *const batch = reinterpret_cast<PPItem *>(wbase + pp_stage_bytes(J) + sizeof(float) * 32 * kLaneFieldsPairs);
+  uint64_t *const bar = reinterpret_cast<uint64_t *>(batch + kPop);
+  uint32_t phase = 0u;
+  bool ok = true;
+  if (lane == 0) {
+    mbar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // ks fields: 0 f2, 1-3 |v| maxima, 4-6 velocity of the owned particle, 7-18 Kahan sums and compensations
+  for (int q = lane; q < J + 32; q += 32) buf[q] = make_float4(0.f, 0.f, 0.f, 0.f);  // always finite
+  for (int f = 0; f < 4; f++) ks[32 * f] = 0.f;
+  __syncwarp();
+  for (int nb = 0, b = 0;; b++) {
+    if (b == nb) {
+      // items [first, last) of tiles [t_lo, t_hi), popped through this launch's own queue head; one at
+      // a time where the items are too few to keep every warp busy otherwise
+      const int32_t *tbase = p.sched + sched_base(p.ntile);
+      const int first = tbase[p.t_lo];
+      const int last = (int)min((int64_t)tbase[p.t_hi], p.item_cap);
+      const int pop = last - first >= 16 * (int)gridDim.x * kPPWarps ? kPop : 1;
+      int it = 0;
+      if (lane == 0) it = first + atomicAdd(p.sched + sched_head(p.ntile, p.t_lo, p.t_hi), pop);
+      it = __shfl_sync(0xffffffffu, it, 0);
+      if (it >= last) break;
+      nb = min(pop, last - it);
+      b = 0;
+      __syncwarp();
+      if (lane < 2 * nb) reinterpret_cast<int4 *>(batch)[lane] = reinterpret_cast<const int4 *>(p.items + it)[lane];
+      __syncwarp();
+    }
+    const PPItem &item = batch[b];  // read from shared memory where used
+    const int ni = item.dims & 0xff;
+    // row r holds particle r mod n2, n2 the power of two from ni up; the 16 / n2 replicas of a particle
+    // take every (16 / n2)-th bit of its lists
+    const int n2 = ni > 8 ? 16 : (ni > 4 ? 8 : (ni > 2 ? 4 : ni));
+    const int iA = g & (n2 - 1), iB = (g + 8) & (n2 - 1);
+    const float4 pA = p.spos[item.i0 + min(iA, ni - 1)], pB = p.spos[item.i0 + min(iB, ni - 1)];
+    // The stencil's rows (dy, dz), one lane each and 32 at a time: every row is a contiguous range of the
+    // cell-sorted particles, and the rows laid end to end are the candidates of the pass.
+    int js = 0, off = 0, walk = 0, r0 = 0;  // this lane's row: first particle, place in the pass; candidates of the pass
+    const int R = (item.dims >> 16) & 0xff, side = 2 * R + 1, nr = side * side;
+    auto load_rows = [&]() {
+      const int ri = r0 + lane;
+      int len = 0;
+      if (ri < nr) {
+        const int q = div_small(ri, side), dz = q - R, dy = ri - q * side - R;
+        if (row_needed(dy, dz, item.h, item.rc2)) {
+          const int S = ((item.dims >> 8) & 0xff) * (p.nt + 2);
+          const int32_t *c = p.cs + ((int)item.cell + (dz * S + dy) * S);
+          js = c[-R];
+          len = c[R + 1 + (item.dims >> 24)] - js;
+        }
+      }
+      int incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      off = incl - len;
+      walk = __shfl_sync(0xffffffffu, incl, 31);
+      r0 += 32;
+    };
+    // Candidates [w, w + n) of the pass into buf[at ..): one bulk copy per row that has some of them
+    // (16-byte entries, so every address and size is a multiple of 16).
+    auto fetch = [&](int w, int n, int at) {
+      const int next = __shfl_down_sync(0xffffffffu, off, 1), end = lane == 31 ? walk : next;
+      const int lo = max(off, w), hi = min(end, w + n);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the warp's own accesses to buf come first
+      __syncwarp();
+      if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)n * 16u);
+      __syncwarp();
+      if (hi > lo) bulk_g2s(buf + at + (lo - w), p.spos + js + (lo - off), (uint32_t)(hi - lo) * 16u, bar);
+    };
+    int w = 0, got = 0;  // candidates of the pass taken so far; those on their way
+    auto request = [&](int room, int at) {  // the next candidates, at most `room` of them; got = 0: the item has no more
+      while (w >= walk) {
+        if (r0 >= nr) {
+          got = 0;
+          return;
+        }
+        load_rows();
+        w = 0;
+      }
+      got = min(walk - w, room);
+      fetch(w, got, at);
+      w += got;
+    };
+    request(J, 0);
+    // the lane that owns a particle: t = 0 the one of row g, t = 1 the one of row g + 8 (when they differ)
+    const bool owner = (t == 0 && g < min(n2, ni)) || (t == 1 && n2 == 16 && g + 8 < ni);
+    const int ip = __float_as_int(t == 1 ? pB.w : pA.w);
+    if (owner) {  // the owned particle's velocity is copied in while the item runs
+      const float *v = p.vp + 3 * (int64_t)ip;
+      cp_async4(ks + 32 * 4, v);
+      cp_async4(ks + 32 * 5, v + 1);
+      cp_async4(ks + 32 * 6, v + 2);
+    }
+    cp_async_commit();
+    // The box of the item's particles: centre and half sides.  Positions are multiples of 2^-17 fine cells
+    // or coarser, so differences to the centre are exact, and so are the differences of two of them.
+    const float lx = warp_min_redux(fminf(pA.x, pB.x)), hx = warp_max_redux(fmaxf(pA.x, pB.x)),
+                ly = warp_min_redux(fminf(pA.y, pB.y)), hy = warp_max_redux(fmaxf(pA.y, pB.y)),
+                lz = warp_min_redux(fminf(pA.z, pB.z)), hz = warp_max_redux(fmaxf(pA.z, pB.z));
+    const float cx = 0.5f * (lx + hx), cy = 0.5f * (ly + hy), cz = 0.5f * (lz + hz);
+    const float ax = fmaxf(hx - cx, cx - lx), ay = fmaxf(hy - cy, cy - ly), az = fmaxf(hz - cz, cz - lz);
+    const float xA = pA.x - cx, yA = pA.y - cy, zA = pA.z - cz;
+    const float xB = pB.x - cx, yB = pB.y - cy, zB = pB.z - cz;
+    // The rows' operand of the filter.  T: rc^2 and the error bound of the product for |x| <= a, |x'| <= m =
+    // a + rc per axis: the rows' values are rounded to 2^-11, the candidates' cut at 2^-10, so at most
+    // 1.5 2^-10 of 2 a m per axis, and 2^-10 of |x'|^2; 5 % and 2e-5 rc^2 cover the FP32 accumulation and
+    // the split of |x|^2 - T.
+    unsigned fa[4];
+    {
+      const float rc = item.rc, mx = ax + rc, my = ay + rc, mz = az + rc;
+      const float T = item.rc2 * 1.00002f +
+                      1.025e-3f * (3.0f * (ax * mx + ay * my + az * mz) + mx * mx + my * my + mz * mz);
+      const float nA = iA < ni ? fmaf(xA, xA, fmaf(yA, yA, zA * zA)) - T : 1e30f;
+      const float nB = iB < ni ? fmaf(xB, xB, fmaf(yB, yB, zB * zB)) - T : 1e30f;
+      const unsigned hA = tf32_floor(nA), hB = tf32_floor(nB);
+      fa[0] = tf32_rna(t == 0 ? -2.0f * xA : (t == 1 ? -2.0f * yA : (t == 2 ? -2.0f * zA : 1.0f)));
+      fa[1] = tf32_rna(t == 0 ? -2.0f * xB : (t == 1 ? -2.0f * yB : (t == 2 ? -2.0f * zB : 1.0f)));
+      fa[2] = t == 0 ? hA : (t == 1 ? tf32_floor(nA - __uint_as_float(hA)) : 0u);
+      fa[3] = t == 0 ? hB : (t == 1 ? tf32_floor(nB - __uint_as_float(hB)) : 0u);
+    }
+    int nflush = 0;
+    float2 px = dup(0.f), py = dup(0.f), pz = dup(0.f);
+    while (got) {
+      int nbuf = 0;  // staged candidates
+      // Candidates farther than rc from the item's box are dropped, in place: what is kept never passes what
+      // has been read.  More are fetched while there is room for a good part of a buffer.
+      do {
+        if (!mbar_wait_bounded(bar, phase)) {
+          ok = false;
+          break;
+        }
+        phase ^= 1u;
+        const int first = nbuf;
+        for (int v = lane; v - lane < got; v += 32) {
+          const float4 pj = buf[first + v];
+          const float qx = pj.x - cx, qy = pj.y - cy, qz = pj.z - cz;
+          const float ex = fmaxf(fabsf(qx) - ax, 0.f), ey = fmaxf(fabsf(qy) - ay, 0.f), ez = fmaxf(fabsf(qz) - az, 0.f);
+          const bool in = (v < got) & (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= item.rc2);
+          const unsigned m = __ballot_sync(0xffffffffu, in);
+          if (in) buf[nbuf + __popc(m & ((1u << lane) - 1u))] = make_float4(qx, qy, qz, fmaf(qx, qx, fmaf(qy, qy, qz * qz)));
+          nbuf += __popc(m);
+        }
+        const bool full = nbuf > J - kRefill;
+        if (full && (w < walk || r0 < nr)) break;
+        request(J - nbuf, nbuf);
+      } while (got);
+      if (!ok) break;
+      // ---- filter: candidate 4 o + t is bit o (from the top) of lane (g, t)'s lists; a step of 8
+      // candidates adds two bits to each list
+      // padding that no row lists; the four candidates after the last step are what an empty list reads
+      if (lane < 16) buf[nbuf + lane] = make_float4(kFar, kFar, kFar, 1e30f);
+      __syncwarp();
+      const int ns = (nbuf + 7) >> 3, c0 = min(ns, 16);
+      unsigned mA0 = 0u, mB0 = 0u, mA1 = 0u, mB1 = 0u;
+      {
+        unsigned sb = buf_s + (unsigned)((4 * (g & 1) + (g >> 1)) * 16 + t * 4);
+        auto filter = [&](int n, unsigned &mA, unsigned &mB) {
+#pragma unroll U
+          for (int s = 0; s < n; s++, sb += 128) {
+            float d[4];
+            mma_tf32(d, fa, tf32_floor(lds32(sb)), __float_as_uint(1.0f));
+            mA = __funnelshift_l(__float_as_uint(d[0]), mA, 1);
+            mA = __funnelshift_l(__float_as_uint(d[1]), mA, 1);
+            mB = __funnelshift_l(__float_as_uint(d[2]), mB, 1);
+            mB = __funnelshift_l(__float_as_uint(d[3]), mB, 1);
+          }
+        };
+        filter(c0, mA0, mB0);
+        filter(ns - c0, mA1, mB1);
+      }
+      if (n2 < 16) {
+        const unsigned every = n2 == 8 ? 0x55555555u : (n2 == 4 ? 0x11111111u : (n2 == 2 ? 0x01010101u : 0x00010001u));
+        const unsigned patA = every << (g / n2), patB = every << ((g + 8) / n2);
+        mA0 &= patA;
+        mA1 &= patA;
+        mB0 &= patB;
+        mB1 &= patB;
+      }
+      const int rounds = __reduce_max_sync(0xffffffffu, max(__popc(mA0) + __popc(mA1), __popc(mB0) + __popc(mB1)));
+      // ---- pairs: bit b of the first list is o = 2 c0 - 1 - b, of the second o = 2 ns - 1 - b
+      unsigned offA = buf_s + (unsigned)(4 * (2 * c0 - 1) + t) * 16u, offB = offA;
+      const unsigned off1 = buf_s + (unsigned)(4 * (2 * ns - 1) + t) * 16u;
+      px = py = pz = dup(0.f);
+      PairLaw law;
+      law.init(item);
+      for (int r = 0; r < rounds; r++) {
+        if (mA0 == 0u) {
+          mA0 = mA1;
+          mA1 = 0u;
+          offA = off1;
+        }
+        if (mB0 == 0u) {
+          mB0 = mB1;
+          mB1 = 0u;
+          offB = off1;
+        }
+        const int bA = high_bit(mA0), bB = high_bit(mB0);
+        const float4 cA = lds128(offA - (unsigned)(bA * 64)), cB = lds128(offB - (unsigned)(bB * 64));
+        mA0 ^= bit_at(bA);
+        mB0 ^= bit_at(bB);
+        const float2 dx = make_float2(cA.x - xA, cB.x - xB), dy = make_float2(cA.y - yA, cB.y - yB),
+                     dz = make_float2(cA.z - zA, cB.z - zB);
+        const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+        float2 s = law.scale2(r2);
+        const bool fA = r2.x > p.app2, fB = r2.y > p.app2;
+        s.x = fA ? s.x : 0.0f;
+        s.y = fB ? s.y : 0.0f;
+        // inside the softening length (rare): both terms directly; r = 0 is the particle itself
+        const bool sA = !fA & (r2.x > 0.0f), sB = !fB & (r2.y > 0.0f);
+        if (sA | sB) {
+          if (sA) s.x = law.soft(r2.x, p.cea, p.ka);
+          if (sB) s.y = law.soft(r2.y, p.cea, p.ka);
+        }
+        px = fma2(s, dx, px);
+        py = fma2(s, dy, py);
+        pz = fma2(s, dz, pz);
+      }
+      nflush++;
+      __syncwarp();
+      const bool more = w < walk || r0 < nr;
+      // compensated sums over the flushes of an item that needs several
+      if (nflush > 1 || more) {
+        const float v[6] = {px.x, py.x, pz.x, px.y, py.y, pz.y};
+#pragma unroll
+        for (int f = 0; f < 6; f++) {
+          if (nflush == 1) {
+            ks[32 * (7 + 2 * f)] = v[f];
+            ks[32 * (8 + 2 * f)] = 0.f;
+          } else {
+            kahan_add(ks[32 * (7 + 2 * f)], ks[32 * (8 + 2 * f)], v[f]);
+          }
+        }
+      }
+      if (more) request(J, 0);
+      else got = 0;
+    }
+    if (!ok) break;
+    // (hi, lo) per half; Kahan c is the negated low part
+    float hi[6] = {px.x, py.x, pz.x, px.y, py.y, pz.y}, lo[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (nflush > 1) {
+#pragma unroll
+      for (int f = 0; f < 6; f++) {
+        hi[f] = ks[32 * (7 + 2 * f)];
+        lo[f] = -ks[32 * (8 + 2 * f)];
+      }
+    }
+    // Sum over the four lanes of a row: lanes of even t keep row g, those of odd t row g + 8, then the
+    // two of a row are joined
+    float H[3], Lo[3];
+#pragma unroll
+    for (int f = 0; f < 3; f++) {
+      const bool odd = t & 1;
+      const float sh = __shfl_xor_sync(0xffffffffu, odd ? hi[f] : hi[3 + f], 1),
+                  sl = __shfl_xor_sync(0xffffffffu, odd ? lo[f] : lo[3 + f], 1);
+      H[f] = odd ? hi[3 + f] : hi[f];
+      Lo[f] = odd ? lo[3 + f] : lo[f];
+      two_sum_merge(H[f], Lo[f], sh, sl);
+    }
+    auto join = [&](int d) {
+#pragma unroll
+      for (int f = 0; f < 3; f++) {
+        const float sh = __shfl_xor_sync(0xffffffffu, H[f], d), sl = __shfl_xor_sync(0xffffffffu, Lo[f], d);
+        two_sum_merge(H[f], Lo[f], sh, sl);
+      }
+    };
+    join(2);
+    if (n2 < 16) {  // the replicas of a particle: row g + 8, and every n2-th row
+      join(1);
+      for (int d = 4 * n2; d < 32; d <<= 1) join(d);
+    }
+    if (owner) {
+      const float fx = (H[0] + Lo[0]) * p.mass2, fy = (H[1] + Lo[1]) * p.mass2, fz = (H[2] + Lo[2]) * p.mass2;
+      ks[0] = fmaxf(ks[0], fx * fx + fy * fy + fz * fz);
+      float *v = p.vp + 3 * (int64_t)ip;
+      cp_async_wait_all();
+      const float v0 = ks[32 * 4] + fx * p.kick, v1 = ks[32 * 5] + fy * p.kick, v2 = ks[32 * 6] + fz * p.kick;
+      v[0] = v0;
+      v[1] = v1;
+      v[2] = v2;
+      ks[32] = fmaxf(ks[32], fabsf(v0));
+      ks[64] = fmaxf(ks[64], fabsf(v1));
+      ks[96] = fmaxf(ks[96], fabsf(v2));
+    }
+    __syncwarp();
+  }
+  if (!ok) {  // a copy did not arrive in time: once more (also bounded), so that none is left behind
+    if (lane == 0) atomicOr(p.err, 1 << CUBE_ERR_TIMEOUT);
+    (void)mbar_wait_bounded(bar, phase);
+    cp_async_wait_all();
+  }
+  const float f2w = warp_max(ks[0]);
+  if (lane == 0) atomic_max_nonneg(&p.out[1], f2w);
+  if (p.want_vmax) {
+    const float vm0 = warp_max(ks[32]), vm1 = warp_max(ks[64]), vm2 = warp_max(ks[96]);
     if (lane == 0) {
       atomic_max_nonneg(&p.out[2], vm0);
       atomic_max_nonneg(&p.out[3], vm1);
@@ -831,7 +1116,6 @@ void launch_pp_items(const PPArgs &a, cudaStream_t s) {
   cudaMemsetAsync(a.sched, 0, sizeof(int32_t) * sched_ints(a.L->ntile), s);
   dim3 grid((unsigned)((p.max_cells + 255) / 256), (unsigned)a.L->ntile);
   switch (pp_shape_desc(a.pairs ? 0 : a.shape).chunk) {
-    case 4: launch_items_c<4>(p, grid, s, a.sched, a.L->ntile); break;
     case 16: launch_items_c<16>(p, grid, s, a.sched, a.L->ntile); break;
     case 32: launch_items_c<32>(p, grid, s, a.sched, a.L->ntile); break;
     default: launch_items_c<8>(p, grid, s, a.sched, a.L->ntile); break;
@@ -843,10 +1127,17 @@ void launch_pp_items(const PPArgs &a, cudaStream_t s) {
 // kernel (slot = shape, or the pair-count kernel) and device: the attribute is per device.
 constexpr int kMaxDevices = 64;
 template <bool COUNT, int S>
+static auto force_kernel() {
+  constexpr PPShapeDesc d = COUNT ? kCountShape : kShapes[S];
+  if constexpr (d.packed != 0) return k_pp_pairs<d.chunk, d.jtile, d.unroll, d.blocks>;
+  else return k_pp_force<COUNT, d.chunk, d.jtile, d.unroll, d.blocks>;
+}
+
+template <bool COUNT, int S>
 static void launch_force_shape(const PPK &p, int num_sms, cudaStream_t s) {
   constexpr PPShapeDesc d = COUNT ? kCountShape : kShapes[S];
   constexpr size_t smem = pp_smem_block(d.jtile, d.packed != 0);
-  auto fn = k_pp_force<COUNT, d.chunk, d.jtile, d.unroll, d.blocks, d.packed != 0>;
+  auto fn = force_kernel<COUNT, S>();
   static int per_sm[kMaxDevices] = {};
   int dev = 0;
   cudaGetDevice(&dev);
