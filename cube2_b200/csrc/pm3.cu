@@ -64,6 +64,19 @@ __device__ __forceinline__ int64_t tsc(double m, float w[3]) {
   return (int64_t)f;
 }
 
+// The same for the brick kernels, whose mesh has a whole number mc <= 16 of points per coarse cell: offset xp of
+// a cell that lies d cells into the brick is the mesh coordinate d mc + (2u + 1) mc / 2^17 from the
+// brick's first owned point.  Its floor and its fraction (17 bits) are exact in integers, so both are
+// those of the real(8) coordinate.
+__device__ __forceinline__ int tsc_brick(int d, int16_t xp, int mc, float w[3]) {
+  const unsigned q = (2u * (uint16_t)xp + 1u) * (unsigned)mc;
+  const float l3 = (float)(q & 0x1ffffu) * (1.0f / 131072.0f);
+  w[0] = __fmul_rn(1.0f - l3, 1.0f - l3) * 0.5f;
+  w[2] = __fmul_rn(l3, l3) * 0.5f;
+  w[1] = 1.0f - w[0] - w[2];
+  return d * mc + (int)(q >> 17);
+}
+
 __global__ void __launch_bounds__(kWarps * 32) k_deposit(PM3K p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t cells = (int64_t)p.rdep[0] * p.rdep[1] * p.rdep[2];
@@ -455,18 +468,20 @@ __device__ __forceinline__ BrickPos brick_pos(const PM3K &p, int64_t b, int cb, 
 // The arithmetic (weights, products, summation order) is the one of k_force_zm followed by
 // k_gather, and the force arrays never reach HBM.
 constexpr int kFgThreads = 1024;
-#ifndef CUBE_FG_PRODUCERS
-#define CUBE_FG_PRODUCERS 512
-#endif
-constexpr int kFgProd = CUBE_FG_PRODUCERS;    // producer threads (the first warps of the block)
+constexpr int kFgProd = 384;                   // producer threads (the first warps of the block)
 constexpr int kFgCons = kFgThreads - kFgProd;  // consumer threads
 static_assert(kFgProd % 32 == 0 && kFgProd >= 128 && kFgCons >= 128, "whole warps in both groups");
 constexpr int kPotX = kBrick + 8, kPotW = kBrick + 6;  // potential window: x 24, y and z 22
-constexpr int kForW = kBrick + 2;                      // force window 18^3
+// force window: y, z the brick and one point on every side, x two (so that pairs of points are aligned)
+constexpr int kForW = kBrick + 2, kForX = kBrick + 4;
 constexpr int kPotElems = kPotW * kPotW * kPotX;
 constexpr uint32_t kPotBytes = sizeof(float) * kPotElems;
-constexpr int kFor3 = kForW * kForW * kForW;
-constexpr size_t kFgSmem = (size_t)kPotBytes + 2 * sizeof(float) * 3 * (size_t)kFor3 + 128;  // + alignment slack
+constexpr int kForElems = kForW * kForW * kForX;
+static_assert(kForElems % 2 == 0 && kPotElems % 4 == 0 && (kForElems + kForElems / 2) % 2 == 0, "16-byte aligned buffers");
+constexpr int kFgMarch = kForW / 2;                        // planes a producer thread marches through
+constexpr int kFgCols = 2 * kForW * (kForX / 2);           // producer threads with work
+static_assert(kFgCols <= kFgProd && kFgMarch * 2 == kForW, "one pass of the producers per brick");
+constexpr size_t kFgSmem = (size_t)kPotBytes + 2 * sizeof(float) * 3 * (size_t)kForElems + 128;  // + alignment slack
 
 struct BrickMeta {
   BrickPos pos;
@@ -520,7 +535,7 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
   extern __shared__ __align__(128) float fg_smem[];
   // the tensor copies land on a 128-byte aligned shared address
   float *pot = fg_smem + ((128u - (smem_addr(fg_smem) & 127u)) & 127u) / 4;  // [z 22][y 22][x 24]
-  float *fwb = pot + kPotElems;                                                 // [2][3][z][y][x] 18^3
+  float2 *fwb = reinterpret_cast<float2 *>(pot + kPotElems);  // [2]: (fx, fy) pairs [z 18][y 18][x 20], then fz
   __shared__ __align__(8) uint64_t bar_pot, bar_full[2], bar_empty[2];
   __shared__ BrickMeta meta[2];
   __shared__ BrickPos s_next;     // the producers' next brick
@@ -529,7 +544,6 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
   __shared__ int s_fail;
   const int tid = threadIdx.x;
   const int cb = kBrick / mc, nrows = cb * cb;
-  const int64_t n = p.n;
   const bool producer = tid < kFgProd;
   const int gt = producer ? tid : tid - kFgProd;  // thread index in the group
   const int lane = tid & 31;
@@ -564,7 +578,8 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
   if (producer) {
     for (int k = 0;; k++) {
       const int b = k & 1;
-      float *fw = fwb + b * 3 * kFor3;
+      float2 *fxy = fwb + b * (kForElems + kForElems / 2);
+      float *fz = reinterpret_cast<float *>(fxy + kForElems);
       BrickMeta &mt = meta[b];
       // the consumers are done with buffer b (brick k - 2)
       bool bad = k >= 2 && !mbar_wait_bounded(&bar_empty[b], (uint32_t)((k - 2) >> 1) & 1u);
@@ -595,18 +610,32 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
         if (lane == 0) mbar_arrive(&bar_full[b]);
         break;
       }
-      constexpr int PY = kPotX, PZ = kPotX * kPotW;
-      for (int e = gt; e < kFor3; e += kFgProd) {
-        const int x = e % kForW, y = (e / kForW) % kForW, z = e / (kForW * kForW);
-        const int c = (z + 2) * PZ + (y + 2) * PY + (x + 3);
-        const float fx = w(pot[c - 2], pot[c - 1], pot[c + 1], pot[c + 2]);
-        const float fy = w(pot[c - 2 * PY], pot[c - PY], pot[c + PY], pot[c + 2 * PY]);
-        const float fz = w(pot[c - 2 * PZ], pot[c - PZ], pot[c + PZ], pot[c + 2 * PZ]);
-        fw[e] = fx;
-        fw[kFor3 + e] = fy;
-        fw[2 * kFor3 + e] = fz;
-        if (x >= 1 && x <= kBrick && y >= 1 && y <= kBrick && z >= 1 && z <= kBrick)
-          m = fmaxf(m, fx * fx + fy * fy + fz * fz);
+      // Thread (x pair, y, half of the planes) marches along z: the five planes of its two points stay in
+      // registers, x and y neighbours are 8-byte reads (7 per two points).
+      if (gt < kFgCols) {
+        const int x2 = gt % (kForX / 2), y = (gt / (kForX / 2)) % kForW, z0 = gt / (kForX / 2 * kForW) * kFgMarch;
+        constexpr int PY = kPotX / 2, PZ = kPotX * kPotW / 2;  // strides of the window in pairs
+        const float2 *c = reinterpret_cast<const float2 *>(pot) + (z0 + 2) * PZ + (y + 2) * PY + (x2 + 1);
+        float2 zm2 = c[-2 * PZ], zm1 = c[-PZ], z0v = c[0], zp1 = c[PZ];
+        const bool own = y >= 1 && y <= kBrick && x2 >= 1 && x2 <= kBrick / 2;  // x window starts two points before the brick
+        int e = (z0 * kForW + y) * kForX + 2 * x2;
+#pragma unroll
+        for (int s = 0; s < kFgMarch; s++, c += PZ, e += kForW * kForX) {
+          const float2 zp2 = c[2 * PZ], xl = c[-1], xr = c[1];
+          const float2 f0 = make_float2(w(xl.x, xl.y, z0v.y, xr.x), w(xl.y, z0v.x, xr.x, xr.y));
+          const float2 a2 = c[-2 * PY], a1 = c[-PY], b1 = c[PY], b2 = c[2 * PY];
+          const float2 f1 = make_float2(w(a2.x, a1.x, b1.x, b2.x), w(a2.y, a1.y, b1.y, b2.y));
+          const float2 f2 = make_float2(w(zm2.x, zm1.x, zp1.x, zp2.x), w(zm2.y, zm1.y, zp1.y, zp2.y));
+          *reinterpret_cast<float4 *>(fxy + e) = make_float4(f0.x, f1.x, f0.y, f1.y);
+          *reinterpret_cast<float2 *>(fz + e) = f2;
+          const int z = z0 + s;
+          if (own && z >= 1 && z <= kBrick)
+            m = fmaxf(m, fmaxf(f0.x * f0.x + f1.x * f1.x + f2.x * f2.x, f0.y * f0.y + f1.y * f1.y + f2.y * f2.y));
+          zm2 = zm1;
+          zm1 = z0v;
+          z0v = zp1;
+          zp1 = zp2;
+        }
       }
       group_any(1, kFgProd, false);  // the window is read, the force buffer and the row counts written
       if (gt == 0) {
@@ -629,7 +658,8 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
   } else {
     for (int k = 0;; k++) {
       const int b = k & 1;
-      const float *fw = fwb + b * 3 * kFor3;
+      const float2 *fxy = fwb + b * (kForElems + kForElems / 2);
+      const float *fz = reinterpret_cast<const float *>(fxy + kForElems);
       const bool bad = !mbar_wait_bounded(&bar_full[b], (uint32_t)(k >> 1) & 1u);
       if (group_any(2, kFgCons, bad)) {
         if (gt == 0) s_fail = 1;
@@ -637,8 +667,6 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
       }
       const BrickMeta &mt = meta[b];
       if (mt.total < 0) break;
-      const BrickPos &q = mt.pos;
-      const MeshJob &J = p.jobs[q.j];
       BrickRows br;
       br.nrows = nrows;
       br.total = mt.total;
@@ -648,24 +676,22 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
         const int64_t ip = brick_particle(kk, br, mt.rbase, mt.rstart, mt.rcell, di, dj, dk);
         const int16_t *qp = p.xp + 3 * ip;
         float wx[3], wy[3], wz[3];
-        const int64_t ix = tsc(decode_pos(q.ci0 + di - p.ncb, qp[0]) * p.scale - J.off[0], wx) + p.shift;
-        const int64_t iy = tsc(decode_pos(q.cj0 + dj - p.ncb, qp[1]) * p.scale - J.off[1], wy) + p.shift;
-        const int64_t iz = tsc(decode_pos(q.ck0 + dk - p.ncb, qp[2]) * p.scale - J.off[2], wz) + p.shift;
-        // the stencil's first point ix - 1 lies at force-window index ix - X0
-        const int lx = (int)wrap_near(ix - q.X0, n), ly = (int)wrap_near(iy - q.Y0, n),
-                  lz = (int)wrap_near(iz - q.Z0, n);
+        // the stencil's first point ix - 1 lies at force-window index (ix - X0) + 1 along x, iy - Y0 along y
+        const int lx = tsc_brick(di, qp[0], mc, wx) + 1, ly = tsc_brick(dj, qp[1], mc, wy),
+                  lz = tsc_brick(dk, qp[2], mc, wz);
         float d0 = 0.f, d1 = 0.f, d2 = 0.f;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
 #pragma unroll
           for (int bb = 0; bb < 3; bb++) {
-            const int row = ((lz + c) * kForW + (ly + bb)) * kForW + lx;
+            const int row = ((lz + c) * kForW + (ly + bb)) * kForX + lx;
 #pragma unroll
             for (int a = 0; a < 3; a++) {
               const float wt = (wx[a] * wy[bb]) * wz[c];
-              d0 += fw[row + a] * wt;
-              d1 += fw[kFor3 + row + a] * wt;
-              d2 += fw[2 * kFor3 + row + a] * wt;
+              const float2 f = fxy[row + a];
+              d0 += f.x * wt;
+              d1 += f.y * wt;
+              d2 += fz[row + a] * wt;
             }
           }
         }
@@ -1118,12 +1144,8 @@ __global__ void __launch_bounds__(kDepThreads) k_deposit_brick(PM3K p, int mc, c
     const int64_t ip = brick_particle(k, br, rbase, rstart, rcell, di, dj, dk);
     const int16_t *qp = p.xp + 3 * ip;
     float wx[3], wy[3], wz[3];
-    const int64_t ix = tsc(decode_pos(q.ci0 + di - p.ncb, qp[0]) * p.scale - J.off[0], wx) + p.shift;
-    const int64_t iy = tsc(decode_pos(q.cj0 + dj - p.ncb, qp[1]) * p.scale - J.off[1], wy) + p.shift;
-    const int64_t iz = tsc(decode_pos(q.ck0 + dk - p.ncb, qp[2]) * p.scale - J.off[2], wz) + p.shift;
     // window indices of the stencil's first point: x (ix - 1) - (X0 - 4), y (iy - 1) - (Y0 - 1)
-    const int lx = (int)wrap_near(ix - q.X0, n) + 3, ly = (int)wrap_near(iy - q.Y0, n),
-              lz = (int)wrap_near(iz - q.Z0, n);
+    const int lx = tsc_brick(di, qp[0], mc, wx) + 3, ly = tsc_brick(dj, qp[1], mc, wy), lz = tsc_brick(dk, qp[2], mc, wz);
     const float sx0 = wx[0] * fs, sx1 = wx[1] * fs, sx2 = wx[2] * fs;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
