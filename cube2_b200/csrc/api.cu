@@ -573,7 +573,8 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
       a.force = (float *)g.force.p;
     } else {
       CK(grow(g.phi_pad, sizeof(float) * m3 * nslots));
-      a.phi_pad = (float *)g.phi_pad.p;
+      a.phi = (float *)g.phi_pad.p;
+      a.phi_pad = kPotPad;
       CK(grow(g.brick_ctr, sizeof(int32_t) * 64));
       a.brick_ctr = (int32_t *)g.brick_ctr.p;
     }
@@ -614,7 +615,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     if (fused) {
       // the potential into the interior of the padded array, then its periodic ghost points
       const int64_t mm = n + 2 * kPotPad;
-      float *interior = a.phi_pad + (kPotPad * mm + kPotPad) * mm + kPotPad;
+      float *interior = a.phi + (kPotPad * mm + kPotPad) * mm + kPotPad;
       if (zsplit) {  // plane transforms, one mesh at a time (the padded meshes are m^3 apart)
         for (int sl = 0; sl < nslots; sl++)
           CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p + (int64_t)sl * nk, (cufftReal *)(interior + sl * mm * mm * mm)));
@@ -651,9 +652,15 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     CU(cudaGetLastError());
     return CUBE_OK;
   }
-  // buffered subtile meshes grouped by level (pm3_fft_cuda.cu:553-591)
-  const size_t soff0 = soff;
+  // Buffered subtile meshes grouped by level (pm3_fft_cuda.cu:553-591), a level in batches of meshes.  The job
+  // tables of all batches go up at once, so that the batches follow one another without a host wait.
   CK(wait_xp(g.stream));
+  struct Batch {
+    int lev, n, nj;
+    size_t job0;
+  };
+  std::vector<Batch> batches;
+  std::vector<MeshJob> jobs;
   for (int lev = 2; lev <= 6; lev++) {
     std::vector<int> locs;
     for (int q = 0; q < L.ns3; q++)
@@ -663,31 +670,19 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     const int rsf = ratio_sf[lev - 1];
     const int nfp = L.ntt * L.rcs * rsf, nfb = L.rcs * rsf, n = nfp + 2 * nfb;
     const int64_t n3 = (int64_t)n * n * n, nk = (int64_t)n * n * (n / 2 + 1);
-    float *G = nullptr;
-    CK(get_green_host(gk[lev - 2], n, &G));
-    const double scale = (double)L.rcs / (double)(1.0f / (float)rsf);
     const size_t per_slot = sizeof(float) * (size_t)n3 * 4 + sizeof(cufftComplex) * (size_t)nk;
     const size_t budget = (size_t)8 << 30;
     int bmax = (int)std::max<size_t>(1, budget / per_slot);
     bmax = std::min<int>(bmax, 512);
     for (size_t j0 = 0; j0 < locs.size(); j0 += bmax) {
       const int nj = (int)std::min<size_t>(bmax, locs.size() - j0);
-      int nb = nj;
-      for (int b : kFftBuckets)
-        if (b >= nj) {
-          nb = b;
-          break;
-        }
-      CK(grow(g.rho, sizeof(float) * n3 * nb));
-      CK(grow(g.rhok, sizeof(cufftComplex) * nk * nb));
-      CK(grow(g.force, sizeof(float) * n3 * 3 * nb));
-      std::vector<MeshJob> jobs(nj);
+      batches.push_back({lev, n, nj, jobs.size()});
       for (int j = 0; j < nj; j++) {
         const int loc = locs[j0 + j];
         const int nss = L.nns * L.nns * L.nns;
         const int t = loc / nss, s = loc % nss;
         const int us[3] = {s % L.nns, (s / L.nns) % L.nns, s / (L.nns * L.nns)};
-        MeshJob &J = jobs[j];
+        MeshJob J;
         J.t = t;
         J.slot = j;
         J.range = 0.f;
@@ -696,54 +691,86 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
           J.alo[q] = us[q] * L.ntt + L.ncb;     // nc1 (kick.f90:503-505)
           J.off[q] = (double)us[q] * nfp;        // utile_shift * nfp (kick.f90:438)
         }
+        jobs.push_back(J);
       }
-      CK(upload(g.jobs, jobs.data(), jobs.size(), soff));
-      PM3Args a{};
-      a.L = &g.L;
-      a.rsf = rsf;
-      a.n = n;
-      a.nslots = nb;
-      a.jobs = (const MeshJob *)g.jobs.p;
-      a.njobs = nj;
-      for (int q = 0; q < 3; q++) {
-        a.rdep[q] = L.ntt + 2;
-        a.ract[q] = L.ntt;
+    }
+  }
+  CK(upload(g.jobs, jobs.data(), jobs.size(), soff));
+  // a stored copy is deposited into the meshes of at most 2 (subtiles of one cell: 3) subtiles per axis
+  const int64_t ndep = d.n_used * (L.ntt > 1 ? 8 : 27);
+  CK(grow(g.dep_items, pm3_dep_items_bytes((int64_t)(L.ntt + 2) * (L.ntt + 2) * (L.ntt + 2), L.ns3, ndep)));
+  CK(grow(g.brick_ctr, sizeof(int32_t) * 64));
+  for (const Batch &bt : batches) {
+    const int rsf = ratio_sf[bt.lev - 1], n = bt.n, nj = bt.nj;
+    const int nfp = L.ntt * L.rcs * rsf, nfb = L.rcs * rsf;
+    const int64_t n3 = (int64_t)n * n * n, nk = (int64_t)n * n * (n / 2 + 1);
+    float *G = nullptr;
+    CK(get_green_host(gk[bt.lev - 2], n, &G));
+    int nb = nj;
+    for (int b : kFftBuckets)
+      if (b >= nj) {
+        nb = b;
+        break;
       }
-      a.wrap = 0;
-      a.shift = nfb;
-      a.fphys_lo = nfb;
-      a.fphys_n = nfp;
-      a.scale = scale;
-      a.xp = d.xp;
-      a.rhoc = d.rhoc;
-      a.cell_base = (const int64_t *)g.cell_base.p;
-      a.rho = (float *)g.rho.p;
-      a.rhok = (cufftComplex *)g.rhok.p;
+    CK(grow(g.rho, sizeof(float) * n3 * nb));
+    CK(grow(g.rhok, sizeof(cufftComplex) * nk * nb));
+    PM3Args a{};
+    a.L = &g.L;
+    a.rsf = rsf;
+    a.n = n;
+    a.nslots = nb;
+    a.jobs = (const MeshJob *)g.jobs.p + bt.job0;
+    a.njobs = nj;
+    for (int q = 0; q < 3; q++) {
+      a.rdep[q] = L.ntt + 2;
+      a.ract[q] = L.ntt;
+    }
+    a.wrap = 0;
+    a.shift = nfb;
+    a.fphys_lo = nfb;
+    a.fphys_n = nfp;
+    a.scale = (double)L.rcs / (double)(1.0f / (float)rsf);
+    a.xp = d.xp;
+    a.rhoc = d.rhoc;
+    a.cell_base = (const int64_t *)g.cell_base.p;
+    a.rho = (float *)g.rho.p;
+    a.rhok = (cufftComplex *)g.rhok.p;
+    a.green = G;
+    a.mass = mass;
+    a.kick = kick;
+    a.vp = d.vp;
+    a.out = (float *)g.out.p;
+    a.want_vmax = want_vmax;
+    a.err = (int32_t *)g.counters.p + 2;
+    a.num_sms = g.num_sms;
+    a.brick_ctr = (int32_t *)g.brick_ctr.p;
+    a.dep_items = (int2 *)g.dep_items.p;
+    a.n_particles_hint = ndep;
+    a.phi = a.rho;  // the potential in place, read by the brick gather where the geometry allows
+    const bool fused = pm3_brick_mc(a) > 0 && nfb >= kPotPad;
+    if (!fused) {
+      CK(grow(g.force, sizeof(float) * n3 * 3 * nb));
       a.force = (float *)g.force.p;
-      a.green = G;
-      a.mass = mass;
-      a.kick = kick;
-      a.vp = d.vp;
-      a.out = (float *)g.out.p;
-      a.want_vmax = want_vmax;
-      cufftHandle fw, bw;
-      CK(get_plan(n, nb, CUFFT_R2C, &fw));
-      CK(get_plan(n, nb, CUFFT_C2R, &bw));
-      CU(cudaMemsetAsync(g.rho.p, 0, sizeof(float) * n3 * nb, g.stream));
-      launch_pm3_deposit(a, g.stream);
-      CF(cufftExecR2C(fw, (cufftReal *)g.rho.p, (cufftComplex *)g.rhok.p));
-      launch_pm3_kspace(a, g.stream);
-      CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)g.rho.p));  // potentials
+    }
+    cufftHandle fw, bw;
+    CK(get_plan(n, nb, CUFFT_R2C, &fw));
+    CK(get_plan(n, nb, CUFFT_C2R, &bw));
+    CU(cudaMemsetAsync(g.rho.p, 0, sizeof(float) * n3 * nb, g.stream));
+    g.launches += launch_pm3_deposit(a, g.stream);
+    CF(cufftExecR2C(fw, (cufftReal *)g.rho.p, (cufftComplex *)g.rhok.p));
+    launch_pm3_kspace(a, g.stream);
+    CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)g.rho.p));  // potentials
+    if (fused) {
+      CK(wait_vp());
+      if (!launch_pm3_force_gather(a, g.stream)) return fail(CUBE_ERR_CUDA);
+    } else {
       a.nslots = nj;  // force and f2max of the real jobs only
       launch_pm3_force(a, g.stream);
       CK(wait_vp());
       launch_pm3_gather(a, g.stream);
-      g.launches += 4;
-      CU(cudaGetLastError());
-      // the job table is reused by the next batch
-      CU(cudaStreamSynchronize(g.stream));
-      soff = soff0;  // tables uploaded before PM3 (the PP grid) keep their staging slots
     }
+    g.launches += fused ? 2 : 3;
+    CU(cudaGetLastError());
   }
   return CUBE_OK;
 }
@@ -981,7 +1008,8 @@ static int run_kick(const int32_t *ires, const int32_t *ixyz3, const int32_t *ra
                     bool do_pp, Meta &m) {
   if (!configured()) return fail(CUBE_ERR_NOT_CONFIGURED);
   CK(build_meta(ires, ixyz3, ratio_sf, apm3, m));
-  CK(stage_begin((size_t)4 << 20));
+  // the subtile geometry uploads one mesh job per subtile
+  CK(stage_begin(((size_t)4 << 20) + (g.L.pm3_mode == CUBE_PM3_SUBTILE ? sizeof(MeshJob) * (size_t)g.L.ns3 : 0)));
   CK(grow(g.cell_base, sizeof(int64_t) * (size_t)g.L.ntile * g.L.nte * g.L.nte * g.L.nte));
   CK(grow(g.out, sizeof(float) * 8));
   CK(grow(g.counters, sizeof(int32_t) * 128));

@@ -253,7 +253,8 @@ struct PM3Args {
   int want_vmax;
   int32_t *err = nullptr;  // device status word (bit CUBE_ERR_TIMEOUT from a bounded wait), may be null
   int num_sms = 148;
-  float *phi_pad = nullptr;  // the potential with kPotPad ghost points per side (periodic images), [nslots][(n+2P)^3]
+  float *phi = nullptr;      // potential of the brick gather, [nslots][(n + 2 phi_pad)^3]
+  int phi_pad = 0;           // its ghost points per side: kPotPad (periodic images), or 0 on buffered meshes
   int32_t *brick_ctr = nullptr;  // work counter of the brick kernels (one int, zeroed by the launcher)
   int2 *dep_items = nullptr;      // deposit work list: pm3_dep_items_bytes(...) of scratch
   int64_t n_particles_hint = 0;   // stored particles (sizes the deposit work list)
@@ -269,11 +270,12 @@ bool pm3_kspace_z_ok(int n);
 void launch_pm3_kspace_z(const PM3Args &a, cudaStream_t s);
 void launch_pm3_force(const PM3Args &a, cudaStream_t s);  // force arrays + f2max from the potential
 void launch_pm3_gather(const PM3Args &a, cudaStream_t s);
-// periodic meshes: the force difference fused into the gather, brick by brick (no force arrays);
-// returns false (nothing launched) where the brick geometry does not apply
+// the force difference fused into the gather, brick by brick (no force arrays); returns false
+// (nothing launched) where the brick geometry does not apply (pm3_brick_mc = 0).  Buffered meshes need
+// at least four buffer points per side
 int pm3_brick_mc(const PM3Args &a);
-bool launch_pm3_force_gather(const PM3Args &a, cudaStream_t s);  // reads a.phi_pad
-void launch_pm3_ghosts(const PM3Args &a, cudaStream_t s);          // fills the ghost points of a.phi_pad
+bool launch_pm3_force_gather(const PM3Args &a, cudaStream_t s);  // reads a.phi
+void launch_pm3_ghosts(const PM3Args &a, cudaStream_t s);          // fills the ghost points of a.phi
 void launch_green_fp64(int n, double apm_soft, double apm_range, double gridsize, int p_order, float *G,
                        cudaStream_t s);
 

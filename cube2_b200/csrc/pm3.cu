@@ -360,34 +360,63 @@ __global__ void __launch_bounds__(kWarps * 32, 4) k_gather(PM3K p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Brick kernels for the periodic meshes (wrap = 1): a brick is kBrick^3 mesh points, i.e.
-// (kBrick / mc)^3 coarse cells of one job, mc = mesh points per coarse cell.  The bricks of a job
-// tile its active cells, and those of all jobs tile the mesh once.  A brick's particles lie in
-// (kBrick / mc)^2 rows of (kBrick / mc) coarse cells, and every row is one contiguous run of
-// storage, so a block walks them as one flat list.
+// Brick kernels: a brick is kBrick^3 mesh points, i.e. (kBrick / mc)^3 coarse cells of one job, mc =
+// mesh points per coarse cell (4, 8 or 16).  The bricks of a job tile its deposited or active
+// cells; where those are no whole number of bricks, the last brick of an axis holds fewer cells.  A
+// brick's particles lie in (kBrick / mc)^2 rows of (kBrick / mc) coarse cells, and every row is one
+// contiguous run of storage, so a block walks them as one flat list.
 constexpr int kBrick = 16;               // owned mesh points per brick side
 constexpr int kMaxCb = 4;                // coarse cells per brick side (mc >= 4)
 constexpr int kMaxRowsPerBrick = kMaxCb * kMaxCb;
 
+// brick b of the launch -> job, first coarse cell, coarse cells a side (fewer than a brick's at the end of
+// a range that is no whole number of bricks), first owned mesh point (exact: the jobs' offsets are
+// whole mesh points, and on buffered meshes the index is in range without wrapping)
+struct BrickPos {
+  int j, ci0, cj0, ck0;
+  int n[3];
+  int64_t X0, Y0, Z0;
+};
+__host__ __device__ __forceinline__ int bricks_of(int ext, int cb) { return (ext + cb - 1) / cb; }
+__device__ __forceinline__ BrickPos brick_pos(const PM3K &p, int64_t b, int cb, const int *ext, const int *lo_of) {
+  const int nbx = bricks_of(ext[0], cb), nby = bricks_of(ext[1], cb), nbz = bricks_of(ext[2], cb);
+  const int64_t per_job = (int64_t)nbx * nby * nbz;
+  BrickPos q;
+  q.j = (int)(b / per_job);
+  const int64_t r = b - (int64_t)q.j * per_job;
+  const MeshJob &J = p.jobs[q.j];
+  const int lo[3] = {lo_of == nullptr ? J.alo[0] : J.lo[0], lo_of == nullptr ? J.alo[1] : J.lo[1],
+                     lo_of == nullptr ? J.alo[2] : J.lo[2]};
+  const int i[3] = {(int)(r % nbx) * cb, (int)((r / nbx) % nby) * cb, (int)(r / ((int64_t)nbx * nby)) * cb};
+  for (int d = 0; d < 3; d++) q.n[d] = min(cb, ext[d] - i[d]);
+  q.ci0 = lo[0] + i[0];
+  q.cj0 = lo[1] + i[1];
+  q.ck0 = lo[2] + i[2];
+  const int64_t n = p.n;
+  q.X0 = wrapi(llrint((double)(q.ci0 - p.ncb) * p.scale - J.off[0]) + p.shift, n);
+  q.Y0 = wrapi(llrint((double)(q.cj0 - p.ncb) * p.scale - J.off[1]) + p.shift, n);
+  q.Z0 = wrapi(llrint((double)(q.ck0 - p.ncb) * p.scale - J.off[2]) + p.shift, n);
+  return q;
+}
+
 struct BrickRows {
   int nrows, total;
-  int cb;  // coarse cells per brick side
+  int cx, cy;  // coarse cells of the brick along x and y
 };
 
 // The brick's rows of coarse cells: first particle, count and the coarse cells' first particles
 // (relative to the row), in shared memory.  Contains two block barriers.
-__device__ __forceinline__ void brick_rows(const PM3K &p, const MeshJob &J, int cb, int ci0, int cj0, int ck0,
-                                          int64_t *rbase, int *rstart, int *rcell, BrickRows &br) {
-  const int nrows = cb * cb;
+__device__ __forceinline__ void brick_rows(const PM3K &p, const MeshJob &J, const BrickPos &q, int64_t *rbase, int *rstart,
+                                          int *rcell, BrickRows &br) {
+  const int nrows = q.n[1] * q.n[2];
   for (int r = threadIdx.x; r < nrows; r += blockDim.x) {
-    const int cj = cj0 + r % cb, ck = ck0 + r / cb;
-    const int64_t c0 = (((int64_t)J.t * p.nte + ck) * p.nte + cj) * p.nte + ci0;
+    const int cj = q.cj0 + r % q.n[1], ck = q.ck0 + r / q.n[1];
+    const int64_t c0 = (((int64_t)J.t * p.nte + ck) * p.nte + cj) * p.nte + q.ci0;
     int acc = 0;
-    for (int i = 0; i < cb; i++) {
+    for (int i = 0; i < q.n[0]; i++) {
       rcell[r * (kMaxCb + 1) + i] = acc;
       acc += p.rhoc[c0 + i];
     }
-    rcell[r * (kMaxCb + 1) + cb] = acc;
     rbase[r] = p.cell_base[c0];
     rstart[r] = acc;  // count for now
   }
@@ -404,7 +433,8 @@ __device__ __forceinline__ void brick_rows(const PM3K &p, const MeshJob &J, int 
   __syncthreads();
   br.nrows = nrows;
   br.total = rstart[nrows];
-  br.cb = cb;
+  br.cx = q.n[0];
+  br.cy = q.n[1];
 }
 
 // Flat particle index k of the brick -> (storage index, coarse cell offsets within the brick).
@@ -417,37 +447,12 @@ __device__ __forceinline__ int64_t brick_particle(int k, const BrickRows &br, co
   }
   const int l = k - rstart[lo];
   int i = 0;
-  while (i + 1 < br.cb && rcell[lo * (kMaxCb + 1) + i + 1] <= l) i++;
+  while (i + 1 < br.cx && rcell[lo * (kMaxCb + 1) + i + 1] <= l) i++;
   di = i;
-  // cb is 1, 2 or 4 (a brick side of 16 mesh points, at least 4 mesh points per coarse cell)
-  dj = lo & (br.cb - 1);
-  dk = lo >> (br.cb >> 1);
+  dk = 0;  // lo = dk cy + dj, with at most kMaxCb rows a side
+  while (lo - dk * br.cy >= br.cy) dk++;
+  dj = lo - dk * br.cy;
   return rbase[lo] + l;
-}
-
-// brick b of the launch -> job, first coarse cell, first owned mesh point (exact: the offsets of
-// periodic jobs are whole mesh points, and the owned points start on a multiple of kBrick)
-struct BrickPos {
-  int j, ci0, cj0, ck0;
-  int64_t X0, Y0, Z0;
-};
-__device__ __forceinline__ BrickPos brick_pos(const PM3K &p, int64_t b, int cb, const int *ext, const int *lo_of) {
-  const int nbx = ext[0] / cb, nby = ext[1] / cb, nbz = ext[2] / cb;
-  const int64_t per_job = (int64_t)nbx * nby * nbz;
-  BrickPos q;
-  q.j = (int)(b / per_job);
-  const int64_t r = b - (int64_t)q.j * per_job;
-  const MeshJob &J = p.jobs[q.j];
-  const int lo[3] = {lo_of == nullptr ? J.alo[0] : J.lo[0], lo_of == nullptr ? J.alo[1] : J.lo[1],
-                     lo_of == nullptr ? J.alo[2] : J.lo[2]};
-  q.ci0 = lo[0] + (int)(r % nbx) * cb;
-  q.cj0 = lo[1] + (int)((r / nbx) % nby) * cb;
-  q.ck0 = lo[2] + (int)(r / ((int64_t)nbx * nby)) * cb;
-  const int64_t n = p.n;
-  q.X0 = wrapi(llrint((double)(q.ci0 - p.ncb) * p.scale - J.off[0]) + p.shift, n);
-  q.Y0 = wrapi(llrint((double)(q.cj0 - p.ncb) * p.scale - J.off[1]) + p.shift, n);
-  q.Z0 = wrapi(llrint((double)(q.ck0 - p.ncb) * p.scale - J.off[2]) + p.shift, n);
-  return q;
 }
 
 // Force and gather in one pass, persistent and warp-specialised: one 1024-thread block per SM
@@ -492,16 +497,15 @@ struct BrickMeta {
 };
 
 // row r of brick (pos) into meta: first particle and the coarse cells' offsets (thread r)
-__device__ __forceinline__ void meta_row(const PM3K &p, int cb, BrickMeta &mt, int r) {
+__device__ __forceinline__ void meta_row(const PM3K &p, BrickMeta &mt, int r) {
   const BrickPos &q = mt.pos;
-  const int cj = q.cj0 + r % cb, ck = q.ck0 + r / cb;
+  const int cj = q.cj0 + r % q.n[1], ck = q.ck0 + r / q.n[1];
   const int64_t c0 = (((int64_t)p.jobs[q.j].t * p.nte + ck) * p.nte + cj) * p.nte + q.ci0;
   int acc = 0;
-  for (int i = 0; i < cb; i++) {
+  for (int i = 0; i < q.n[0]; i++) {
     mt.rcell[r * (kMaxCb + 1) + i] = acc;
     acc += p.rhoc[c0 + i];
   }
-  mt.rcell[r * (kMaxCb + 1) + cb] = acc;
   mt.rbase[r] = p.cell_base[c0];
   mt.rstart[r] = acc;  // count until meta_scan
 }
@@ -530,7 +534,7 @@ __device__ __forceinline__ bool group_any(int id, int count, bool v) {
   return r != 0;
 }
 
-__global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, int64_t nbricks,
+__global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, int64_t nbricks, int pad,
                                                                 const __grid_constant__ CUtensorMap tmap) {
   extern __shared__ __align__(128) float fg_smem[];
   // the tensor copies land on a 128-byte aligned shared address
@@ -543,14 +547,14 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
   __shared__ float red[4][kFgThreads / 32];
   __shared__ int s_fail;
   const int tid = threadIdx.x;
-  const int cb = kBrick / mc, nrows = cb * cb;
+  const int cb = kBrick / mc;
   const bool producer = tid < kFgProd;
   const int gt = producer ? tid : tid - kFgProd;  // thread index in the group
   const int lane = tid & 31;
   if (blockIdx.x >= nbricks) return;
   auto request = [&](const BrickPos &q) {  // thread 0: the potential window of brick q
     mbar_arrive_expect_tx(&bar_pot, kPotBytes);  // the phase completes when the bytes have landed
-    const int cx = (int)q.X0 - 4 + kPotPad, cy = (int)q.Y0 - 3 + kPotPad, cz = (int)q.Z0 - 3 + kPotPad;
+    const int cx = (int)q.X0 - 4 + pad, cy = (int)q.Y0 - 3 + pad, cz = (int)q.Z0 - 3 + pad;
     const int cs = p.jobs[q.j].slot;
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
@@ -597,7 +601,8 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
       }
       if (gt == 0) mt.pos = s_next;
       group_any(1, kFgProd, false);  // mt.pos visible to the group
-      if (gt < nrows) meta_row(p, cb, mt, gt);
+      const int nrows = mt.pos.n[1] * mt.pos.n[2];
+      if (gt < nrows) meta_row(p, mt, gt);
       // this brick's potential window
       bad = !mbar_wait_bounded(&bar_pot, (uint32_t)nok & 1u);
       if (!bad) nok++;
@@ -617,7 +622,9 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
         constexpr int PY = kPotX / 2, PZ = kPotX * kPotW / 2;  // strides of the window in pairs
         const float2 *c = reinterpret_cast<const float2 *>(pot) + (z0 + 2) * PZ + (y + 2) * PY + (x2 + 1);
         float2 zm2 = c[-2 * PZ], zm1 = c[-PZ], z0v = c[0], zp1 = c[PZ];
-        const bool own = y >= 1 && y <= kBrick && x2 >= 1 && x2 <= kBrick / 2;  // x window starts two points before the brick
+        // owned points (the x window starts two points before the brick's, y and z windows one)
+        const int ox = mt.pos.n[0] * mc, oy = mt.pos.n[1] * mc, oz = mt.pos.n[2] * mc;
+        const bool own = y >= 1 && y <= oy && x2 >= 1 && 2 * x2 <= ox;
         int e = (z0 * kForW + y) * kForX + 2 * x2;
 #pragma unroll
         for (int s = 0; s < kFgMarch; s++, c += PZ, e += kForW * kForX) {
@@ -629,7 +636,7 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
           *reinterpret_cast<float4 *>(fxy + e) = make_float4(f0.x, f1.x, f0.y, f1.y);
           *reinterpret_cast<float2 *>(fz + e) = f2;
           const int z = z0 + s;
-          if (own && z >= 1 && z <= kBrick)
+          if (own && z >= 1 && z <= oz)
             m = fmaxf(m, fmaxf(f0.x * f0.x + f1.x * f1.x + f2.x * f2.x, f0.y * f0.y + f1.y * f1.y + f2.y * f2.y));
           zm2 = zm1;
           zm1 = z0v;
@@ -668,9 +675,10 @@ __global__ void __launch_bounds__(kFgThreads, 1) k_force_gather(PM3K p, int mc, 
       const BrickMeta &mt = meta[b];
       if (mt.total < 0) break;
       BrickRows br;
-      br.nrows = nrows;
+      br.nrows = mt.pos.n[1] * mt.pos.n[2];
       br.total = mt.total;
-      br.cb = cb;
+      br.cx = mt.pos.n[0];
+      br.cy = mt.pos.n[1];
       for (int kk = gt; kk < br.total; kk += kFgCons) {
         int di, dj, dk;
         const int64_t ip = brick_particle(kk, br, mt.rbase, mt.rstart, mt.rcell, di, dj, dk);
@@ -1082,6 +1090,7 @@ void launch_pm3_force(const PM3Args &a, cudaStream_t s) {
 // independent of the order of the atomics (the rounding of a weight to 2^-e, e >= 15 for
 // bricks of up to 10^5 particles, is far below the FP32 rounding of the density).
 constexpr int kDepThreads = 256;
+constexpr int kDepBlocks = 5;  // resident blocks per SM (48 registers a thread)
 constexpr int kAccX = kBrick + 8;  // x window owned - 4 .. owned + kBrick + 3: whole float4 groups
 constexpr int kAccW = kBrick + 2;  // y, z window owned - 1 .. owned + kBrick
 
@@ -1097,10 +1106,10 @@ __global__ void k_dep_items(PM3K p, int mc, int64_t nbricks, int chunk, int2 *it
     const BrickPos q = brick_pos(p, b, cb, p.rdep, p.rdep);
     const int64_t t = p.jobs[q.j].t;
     int total = 0;
-    for (int k = 0; k < cb; k++)
-      for (int j = 0; j < cb; j++) {
+    for (int k = 0; k < q.n[2]; k++)
+      for (int j = 0; j < q.n[1]; j++) {
         const int32_t *r = p.rhoc + ((t * p.nte + q.ck0 + k) * p.nte + q.cj0 + j) * p.nte + q.ci0;
-        for (int i = 0; i < cb; i++) total += r[i];
+        for (int i = 0; i < q.n[0]; i++) total += r[i];
       }
     if (total == 0) continue;
     const int nch = min((total + chunk - 1) / chunk, 0x7fff);
@@ -1113,87 +1122,89 @@ __global__ void k_dep_items(PM3K p, int mc, int64_t nbricks, int chunk, int2 *it
   }
 }
 
-__global__ void __launch_bounds__(kDepThreads) k_deposit_brick(PM3K p, int mc, const int2 *items, const int *count) {
+__global__ void __launch_bounds__(kDepThreads, kDepBlocks) k_deposit_brick(PM3K p, int mc, const int2 *items,
+                                                                               const int *count, int cap) {
   __shared__ __align__(16) unsigned acc[kAccW * kAccW * kAccX];
   __shared__ int64_t rbase[kMaxRowsPerBrick];
   __shared__ int rstart[kMaxRowsPerBrick + 1];
   __shared__ int rcell[kMaxRowsPerBrick * (kMaxCb + 1)];
-  int2 item = make_int2((int)blockIdx.x, 1 << 16);  // without a work list: one block per whole brick
-  if (items) {
-    if ((int)blockIdx.x >= min(*count, (int)gridDim.x)) return;
-    item = items[blockIdx.x];
-  }
-  const int chunk = item.y & 0xffff, nch = item.y >> 16;
-  const int cb = kBrick / mc;
-  const BrickPos q = brick_pos(p, item.x, cb, p.rdep, p.rdep);
-  const MeshJob &J = p.jobs[q.j];
-  const int64_t n = p.n;
-  for (int e4 = threadIdx.x; e4 < kAccW * kAccW * kAccX / 4; e4 += kDepThreads)
-    reinterpret_cast<uint4 *>(acc)[e4] = make_uint4(0u, 0u, 0u, 0u);
-  BrickRows br;
-  brick_rows(p, J, cb, q.ci0, q.cj0, q.ck0, rbase, rstart, rcell, br);  // its barriers cover the zeroing
-  // this item's particles of the brick
-  const int k0 = (int)((int64_t)br.total * chunk / nch), k1 = (int)((int64_t)br.total * (chunk + 1) / nch);
-  if (k1 <= k0) return;
-  // fixed-point scale 2^e: particles * 0.4219 * 2^e < 2^32
-  int e = 24;
-  while (e > 1 && (double)(k1 - k0) * 0.421875 * (double)(1u << e) >= 4294967040.0) e--;
-  const float fs = (float)(1u << e), inv = 1.0f / fs;
-  for (int k = k0 + threadIdx.x; k < k1; k += kDepThreads) {
-    int di, dj, dk;
-    const int64_t ip = brick_particle(k, br, rbase, rstart, rcell, di, dj, dk);
-    const int16_t *qp = p.xp + 3 * ip;
-    float wx[3], wy[3], wz[3];
-    // window indices of the stencil's first point: x (ix - 1) - (X0 - 4), y (iy - 1) - (Y0 - 1)
-    const int lx = tsc_brick(di, qp[0], mc, wx) + 3, ly = tsc_brick(dj, qp[1], mc, wy), lz = tsc_brick(dk, qp[2], mc, wz);
-    const float sx0 = wx[0] * fs, sx1 = wx[1] * fs, sx2 = wx[2] * fs;
+  // items one after the other, a block taking every gridDim.x-th; without a work list a whole brick each
+  const int n_items = items ? min(*count, cap) : cap;
+  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+    const int2 item = items ? items[it] : make_int2(it, 1 << 16);
+    const int chunk = item.y & 0xffff, nch = item.y >> 16;
+    const int cb = kBrick / mc;
+    const BrickPos q = brick_pos(p, item.x, cb, p.rdep, p.rdep);
+    const MeshJob &J = p.jobs[q.j];
+    for (int e4 = threadIdx.x; e4 < kAccW * kAccW * kAccX / 4; e4 += kDepThreads)
+      reinterpret_cast<uint4 *>(acc)[e4] = make_uint4(0u, 0u, 0u, 0u);
+    BrickRows br;
+    brick_rows(p, J, q, rbase, rstart, rcell, br);  // its barriers cover the zeroing
+    // this item's particles of the brick
+    const int k0 = (int)((int64_t)br.total * chunk / nch), k1 = (int)((int64_t)br.total * (chunk + 1) / nch);
+    if (k1 <= k0) {  // the same for the whole block; the next item rewrites the row tables
+      __syncthreads();
+      continue;
+    }
+    // fixed-point scale 2^e: particles * 0.4219 * 2^e < 2^32
+    int e = 24;
+    while (e > 1 && (double)(k1 - k0) * 0.421875 * (double)(1u << e) >= 4294967040.0) e--;
+    const float fs = (float)(1u << e), inv = 1.0f / fs;
+    for (int k = k0 + threadIdx.x; k < k1; k += kDepThreads) {
+      int di, dj, dk;
+      const int64_t ip = brick_particle(k, br, rbase, rstart, rcell, di, dj, dk);
+      const int16_t *qp = p.xp + 3 * ip;
+      float wx[3], wy[3], wz[3];
+      // window indices of the stencil's first point: x (ix - 1) - (X0 - 4), y (iy - 1) - (Y0 - 1)
+      const int lx = tsc_brick(di, qp[0], mc, wx) + 3, ly = tsc_brick(dj, qp[1], mc, wy), lz = tsc_brick(dk, qp[2], mc, wz);
+      const float sx0 = wx[0] * fs, sx1 = wx[1] * fs, sx2 = wx[2] * fs;
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
+      for (int c = 0; c < 3; c++) {
 #pragma unroll
-      for (int bb = 0; bb < 3; bb++) {
-        unsigned *row = acc + ((lz + c) * kAccW + (ly + bb)) * kAccX + lx;
-        const float yz = wy[bb] * wz[c];
-        atomicAdd(row + 0, __float2uint_rn(sx0 * yz));
-        atomicAdd(row + 1, __float2uint_rn(sx1 * yz));
-        atomicAdd(row + 2, __float2uint_rn(sx2 * yz));
+        for (int bb = 0; bb < 3; bb++) {
+          unsigned *row = acc + ((lz + c) * kAccW + (ly + bb)) * kAccX + lx;
+          const float yz = wy[bb] * wz[c];
+          atomicAdd(row + 0, __float2uint_rn(sx0 * yz));
+          atomicAdd(row + 1, __float2uint_rn(sx1 * yz));
+          atomicAdd(row + 2, __float2uint_rn(sx2 * yz));
+        }
       }
     }
-  }
-  __syncthreads();
-  // Flush: lane (w, xg) of a warp takes x group xg (lane % 6) of window rows 5 pass + w (w < 5), so
-  // the group's mesh x index is worked out once and each row's once per pass.
-  float *R = p.rho + (int64_t)J.slot * p.n3;
-  constexpr int G4 = kAccX / 4, kRowsPerWarp = 32 / G4, kRows = kAccW * kAccW;
-  const int lane = threadIdx.x & 31, w = lane / G4, xg = lane - w * G4;
-  if (w < kRowsPerWarp) {
-    const int ni = (int)n;
-    auto wrap32 = [ni](int a) { return a < 0 ? a + ni : (a >= ni ? a - ni : a); };
-    const int gx = wrap32((int)q.X0 - 4 + 4 * xg);
-    for (int row = (threadIdx.x >> 5) * kRowsPerWarp + w; row < kRows; row += (kDepThreads / 32) * kRowsPerWarp) {
-      const uint4 u = reinterpret_cast<const uint4 *>(acc)[row * G4 + xg];
-      if ((u.x | u.y | u.z | u.w) == 0u) continue;
-      const int gy = wrap32((int)q.Y0 - 1 + row % kAccW), gz = wrap32((int)q.Z0 - 1 + row / kAccW);
-      atomicAdd(reinterpret_cast<float4 *>(R + ((int64_t)gz * ni + gy) * ni + gx),
-                make_float4((float)u.x * inv, (float)u.y * inv, (float)u.z * inv, (float)u.w * inv));
+    __syncthreads();
+    // Flush: lane (w, xg) of a warp takes x group xg (lane % 6) of window rows 5 pass + w (w < 5), so
+    // the group's mesh x index is worked out once and each row's once per pass.
+    float *R = p.rho + (int64_t)J.slot * p.n3;
+    constexpr int G4 = kAccX / 4, kRowsPerWarp = 32 / G4, kRows = kAccW * kAccW;
+    const int lane = threadIdx.x & 31, w = lane / G4, xg = lane - w * G4;
+    if (w < kRowsPerWarp) {
+      // periodic meshes wrap; buffered ones drop what lies outside (-1), as kick.f90:448-466 does
+      const int ni = p.n, wrapped = p.wrap ? ni : 0;
+      auto place = [ni, wrapped](int a) {
+        a += a < 0 ? wrapped : (a >= ni ? -wrapped : 0);
+        return a >= ni ? -1 : a;
+      };
+      const int gx = place((int)q.X0 - 4 + 4 * xg);
+      for (int row = (threadIdx.x >> 5) * kRowsPerWarp + w; row < kRows; row += (kDepThreads / 32) * kRowsPerWarp) {
+        const uint4 u = reinterpret_cast<const uint4 *>(acc)[row * G4 + xg];
+        if ((u.x | u.y | u.z | u.w) == 0u) continue;
+        const int gy = place((int)q.Y0 - 1 + row % kAccW), gz = place((int)q.Z0 - 1 + row / kAccW);
+        if ((gx | gy | gz) < 0) continue;
+        atomicAdd(reinterpret_cast<float4 *>(R + ((int64_t)gz * ni + gy) * ni + gx),
+                  make_float4((float)u.x * inv, (float)u.y * inv, (float)u.z * inv, (float)u.w * inv));
+      }
     }
+    __syncthreads();  // the window is read: the next item may clear it
   }
 }
 
-// mesh points per coarse cell when the brick kernels apply (periodic meshes, whole mesh points
-// per coarse cell dividing the brick, the deposited (dep) or gathered cells of every job a whole
-// number of bricks), else 0
-static int brick_mc(const PM3Args &a, bool dep) {
-  if (!a.wrap || a.n < 8) return 0;
-  const double mcd = a.scale;
-  const int mc = (int)llrint(mcd);
-  if (mc < 1 || (double)mc != mcd || kBrick % mc) return 0;
-  const int cb = kBrick / mc;
-  if (cb > kMaxCb) return 0;
-  for (int d = 0; d < 3; d++)
-    if ((dep ? a.rdep[d] : a.ract[d]) % cb) return 0;
-  return mc;
+// mesh points per coarse cell when the brick kernels apply (4, 8 or 16 exactly, on rows of whole 16-byte
+// groups), else 0
+int pm3_brick_mc(const PM3Args &a) {
+  const int mc = (int)llrint(a.scale);
+  if ((double)mc != a.scale || (mc != 4 && mc != 8 && mc != 16)) return 0;
+  static_assert(kBrick / 4 <= kMaxCb && kBrick % 16 == 0, "whole coarse cells per brick");
+  return a.n >= 16 && a.n % 4 == 0 && a.shift % 4 == 0 ? mc : 0;
 }
-int pm3_brick_mc(const PM3Args &a) { return brick_mc(a, false); }
 
 // the dynamic shared-memory limit of a kernel, raised once per device (the attribute is per device)
 static void set_smem_attr_once(const void *fn, size_t bytes) {
@@ -1221,15 +1232,16 @@ size_t pm3_dep_items_bytes(int64_t cells_per_job, int njobs, int64_t n_used) {
 
 int launch_pm3_deposit(const PM3Args &a, cudaStream_t s) {
   PM3K p = make_k(a);
-  const int mc = (a.n % 4 == 0) ? brick_mc(a, true) : 0;
+  const int mc = pm3_brick_mc(a);
   if (mc) {
     constexpr int chunk = kDepChunk;
     auto kern = k_deposit_brick;
     const int cb = kBrick / mc;
-    const int64_t nbricks = (int64_t)(a.rdep[0] / cb) * (a.rdep[1] / cb) * (a.rdep[2] / cb) * a.njobs;
+    const int64_t nbricks = (int64_t)bricks_of(a.rdep[0], cb) * bricks_of(a.rdep[1], cb) * bricks_of(a.rdep[2], cb) * a.njobs;
     if (nbricks <= 0) return 0;
+    const int64_t resident = (int64_t)(a.num_sms > 0 ? a.num_sms : 148) * kDepBlocks;
     if (!a.dep_items) {
-      kern<<<(unsigned)nbricks, kDepThreads, 0, s>>>(p, mc, nullptr, nullptr);
+      kern<<<(unsigned)std::min(nbricks, resident), kDepThreads, 0, s>>>(p, mc, nullptr, nullptr, (int)nbricks);
       return 1;
     }
     // at most one item per brick plus one per `chunk` particles
@@ -1238,7 +1250,7 @@ int launch_pm3_deposit(const PM3Args &a, cudaStream_t s) {
     cudaMemsetAsync(count, 0, sizeof(int), s);
     k_dep_items<<<(unsigned)std::min<int64_t>((nbricks + 255) / 256, 4096), 256, 0, s>>>(p, mc, nbricks, chunk,
                                                                                        a.dep_items, count, cap);
-    kern<<<(unsigned)cap, kDepThreads, 0, s>>>(p, mc, a.dep_items, count);
+    kern<<<(unsigned)std::min(cap, resident), kDepThreads, 0, s>>>(p, mc, a.dep_items, count, (int)cap);
     return 2;
   }
   const int64_t warps = (int64_t)a.rdep[0] * a.rdep[1] * a.rdep[2] * a.njobs;
@@ -1262,29 +1274,29 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 bool launch_pm3_force_gather(const PM3Args &a, cudaStream_t s) {
-  const int mc = brick_mc(a, false);
-  if (!mc || !a.phi_pad) return false;
+  const int mc = pm3_brick_mc(a);
+  if (!mc || !a.phi) return false;
   PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (!encode) return false;
-  // the padded potential as a 4-d tensor [slot][z][y][x], boxes of the potential window
-  const cuuint64_t m = (cuuint64_t)a.n + 2 * kPotPad;
+  // the potential as a 4-d tensor [slot][z][y][x], boxes of the potential window
+  const cuuint64_t m = (cuuint64_t)a.n + 2 * a.phi_pad;
   const cuuint64_t dims[4] = {m, m, m, (cuuint64_t)a.nslots};
   const cuuint64_t strides[3] = {m * 4, m * m * 4, m * m * m * 4};
   const cuuint32_t box[4] = {kPotX, kPotW, kPotW, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUtensorMap tmap;
-  if (encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.phi_pad, dims, strides, box, estr,
+  if (encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.phi, dims, strides, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
   PM3K p = make_k(a);
   const int cb = kBrick / mc;
-  const int64_t nbricks = (int64_t)(a.ract[0] / cb) * (a.ract[1] / cb) * (a.ract[2] / cb) * a.njobs;
+  const int64_t nbricks = (int64_t)bricks_of(a.ract[0], cb) * bricks_of(a.ract[1], cb) * bricks_of(a.ract[2], cb) * a.njobs;
   set_smem_attr_once((const void *)k_force_gather, kFgSmem);
   const int64_t grid = std::min<int64_t>(nbricks, a.num_sms > 0 ? a.num_sms : 148);
   if (!a.brick_ctr) return false;
   cudaMemsetAsync(a.brick_ctr, 0, sizeof(int32_t), s);
-  if (grid > 0) k_force_gather<<<(unsigned)grid, kFgThreads, kFgSmem, s>>>(p, mc, nbricks, tmap);
+  if (grid > 0) k_force_gather<<<(unsigned)grid, kFgThreads, kFgSmem, s>>>(p, mc, nbricks, a.phi_pad, tmap);
   return true;
 }
 
@@ -1325,11 +1337,10 @@ __global__ void k_pm3_ghosts(float *phi, int n, int nslots) {
 }
 
 void launch_pm3_ghosts(const PM3Args &a, cudaStream_t s) {
-  if (!a.phi_pad) return;
   const int m = a.n + 2 * kPotPad;
   const int64_t per = (int64_t)2 * kPotPad * m * m + (int64_t)a.n * 2 * kPotPad * m + (int64_t)a.n * a.n * 2 * kPotPad;
   const unsigned gx = (unsigned)std::min<int64_t>((per + 255) / 256, 4096);
-  k_pm3_ghosts<<<dim3(gx, (unsigned)a.nslots), 256, 0, s>>>(a.phi_pad, a.n, a.nslots);
+  k_pm3_ghosts<<<dim3(gx, (unsigned)a.nslots), 256, 0, s>>>(a.phi, a.n, a.nslots);
 }
 
 void launch_pm3_gather(const PM3Args &a, cudaStream_t s) {
