@@ -50,6 +50,8 @@ struct DriftK {
   int64_t n_used, n_used_new;  // stored copies of the current / new image (bounds of the spines)
   float dt_mid, rcs_f;
   double xres_rcs;     // x_resolution * ratio_cs
+  float inv_rcs;       // 1 / ratio_cs where that is a power of two (then a product is the quotient bit for bit), else 0
+  double inv_xres_rcs;
   const int32_t *rhoc;
   const int64_t *cell_base;
   const int16_t *xp;
@@ -74,33 +76,56 @@ struct DriftK {
   int64_t *pid_new;
 };
 
+// 32-bit arithmetic: the images have fewer than 2^31 extended cells, and a 64-bit division is a long software
+// sequence that every warp would run for each of its cells (k_halo_fill took 73 us on 256^3, most of it this)
 __device__ __forceinline__ void cell_of(const DriftK &p, int64_t S, int &t, int &cx, int &cy, int &cz) {
-  const int64_t n3 = (int64_t)p.nte * p.nte * p.nte;
-  t = (int)(S / n3);
-  int64_t r = S - (int64_t)t * n3;
-  cz = (int)(r / (p.nte * p.nte));
-  r -= (int64_t)cz * p.nte * p.nte;
-  cy = (int)(r / p.nte);
-  cx = (int)(r - (int64_t)cy * p.nte);
+  const unsigned n = (unsigned)p.nte, q = (unsigned)S / n, qq = q / n;
+  cx = (int)((unsigned)S - q * n);
+  cy = (int)(q - qq * n);
+  t = (int)(qq / n);
+  cz = (int)(qq - (unsigned)t * n);
 }
 
 // drift.f90:57-66: destination of a stored copy, or -1 when it leaves the tile's physical
 // region.  xq = (i-1) + (u+0.5) 2^-16 is exact in double; deltax = (dt_mid*vp)/ratio_cs
 // in float; ig = ceiling(xq + deltax) in [1, nt] <=> 0 < xq + deltax <= nt.
-__device__ __forceinline__ int32_t drift_dest(const DriftK &p, int64_t ip, int cx, int cy, int cz, int t) {
-  const int c[3] = {cx, cy, cz};
-  const int tt[3] = {t % p.nnt, (t / p.nnt) % p.nnt, t / (p.nnt * p.nnt)};
+struct DriftCell {
+  int c[3];  // coarse coordinates in the tile, -ncb .. nt + ncb - 1
+  int o[3];  // image coordinates of the tile's first physical cell
+};
+__device__ __forceinline__ DriftCell drift_cell(const DriftK &p, int64_t S, int &cz) {
+  DriftCell q;
+  int t, cx, cy;
+  cell_of(p, S, t, cx, cy, cz);
+  const int ty = t / p.nnt, tz = ty / p.nnt;
+  q.c[0] = cx - p.ncb;
+  q.c[1] = cy - p.ncb;
+  q.c[2] = cz - p.ncb;
+  q.o[0] = (t - ty * p.nnt) * p.nt;
+  q.o[1] = (ty - tz * p.nnt) * p.nt;
+  q.o[2] = tz * p.nt;
+  return q;
+}
+__device__ __forceinline__ int32_t drift_dest(const DriftK &p, int64_t ip, const DriftCell &q) {
   int g[3];
+  float v[3];
+  uint16_t u[3];
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    const double frac = ((double)(uint16_t)p.xp[3 * ip + d] + 0.5) * (1.0 / 65536.0);
-    const double xq = (double)(c[d] - p.ncb) + frac;
-    const float dl = __fdiv_rn(__fmul_rn(p.dt_mid, p.vp[3 * ip + d]), p.rcs_f);
-    const double s = __dadd_rn(xq, (double)dl);
-    if (!(s > 0.0 && s <= (double)p.nt)) return -1;
-    g[d] = tt[d] * p.nt + (int)ceil(s) - 1;
+    v[d] = p.vp[3 * ip + d];
+    u[d] = (uint16_t)p.xp[3 * ip + d];
   }
-  return (g[2] * p.nc + g[1]) * p.nc + g[0];
+  bool in = true;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const double xq = (double)q.c[d] + ((double)u[d] + 0.5) * (1.0 / 65536.0);
+    const float dv = __fmul_rn(p.dt_mid, v[d]);
+    const float dl = p.inv_rcs != 0.f ? __fmul_rn(dv, p.inv_rcs) : __fdiv_rn(dv, p.rcs_f);
+    const double s = __dadd_rn(xq, (double)dl);
+    in = in && s > 0.0 && s <= (double)p.nt;
+    g[d] = q.o[d] + (in ? __double2int_ru(s) - 1 : 0);
+  }
+  return in ? (g[2] * p.nc + g[1]) * p.nc + g[0] : -1;
 }
 
 __global__ void __launch_bounds__(kDriftWarps * 32) k_drift_runs(DriftK p) {
@@ -136,19 +161,37 @@ __global__ void __launch_bounds__(kDriftWarps * 32) k_drift_runs(DriftK p) {
       if (lane == 0) atomicOr(p.err, 1 << CUBE_ERR_INVALID);
       continue;
     }
-    int t, cx, cy, cz;
-    cell_of(p, S, t, cx, cy, cz);
+    int cz;
+    const DriftCell cell = drift_cell(p, S, cz);
     int nent = 0;  // warp-uniform
+    // most copies stay in their own cell: its run is counted in registers, without the search
+    const bool phys = cell.c[0] >= 0 && cell.c[0] < p.nt && cell.c[1] >= 0 && cell.c[1] < p.nt && cell.c[2] >= 0 &&
+                      cell.c[2] < p.nt;
+    const int32_t home =
+        phys ? ((cell.o[2] + cell.c[2]) * p.nc + cell.o[1] + cell.c[1]) * p.nc + cell.o[0] + cell.c[0] : -2;
+    int ehome = -1, nhome = 0;  // entry and copies of that run
     // 64 copies per step: the loads of both halves are in flight together
     for (int c64 = 0; c64 < n; c64 += 64) {
-    const int32_t D2[2] = {c64 + lane < n ? drift_dest(p, base + c64 + lane, cx, cy, cz, t) : -1,
-                           c64 + 32 + lane < n ? drift_dest(p, base + c64 + 32 + lane, cx, cy, cz, t) : -1};
+    const int32_t D2[2] = {c64 + lane < n ? drift_dest(p, base + c64 + lane, cell) : -1,
+                           c64 + 32 + lane < n ? drift_dest(p, base + c64 + 32 + lane, cell) : -1};
     for (int h = 0; h < 2 && c64 + 32 * h < n; h++) {
       const int c0 = c64 + 32 * h;
       const int l = c0 + lane;
       const int32_t D = D2[h];
       uint32_t word = kDropped;
-      unsigned pending = __ballot_sync(0xffffffffu, D >= 0);
+      const unsigned hm = __ballot_sync(0xffffffffu, D == home);
+      if (hm && ehome < 0) {
+        if (nent < kDriftMaxRuns) {
+          ehome = nent++;
+          if (lane == 0) td[ehome] = home;
+          __syncwarp();
+        } else if (lane == 0) {
+          atomicOr(p.err, 1 << CUBE_ERR_CAPACITY);
+        }
+      }
+      if (ehome >= 0 && D == home) word = ((uint32_t)ehome << kRankBits) | (uint32_t)(nhome + __popc(hm & lt));
+      nhome += __popc(hm);
+      unsigned pending = __ballot_sync(0xffffffffu, D >= 0) & ~hm;
       while (pending) {
         const int32_t Dl = __shfl_sync(0xffffffffu, D, __ffs(pending) - 1);
         const unsigned grp = __ballot_sync(0xffffffffu, D == Dl);
@@ -176,6 +219,10 @@ __global__ void __launch_bounds__(kDriftWarps * 32) k_drift_runs(DriftK p) {
       }
       if (l < n) p.runrank[base + l] = word;
     }
+    }
+    if (ehome >= 0) {
+      if (lane == 0) tc[ehome] = nhome;
+      __syncwarp();
     }
     if (nent) {
       if (cur + nent > end) {  // a new chunk of run slots
@@ -214,39 +261,52 @@ __global__ void __launch_bounds__(kDriftWarps * 32) k_drift_runs(DriftK p) {
 }
 
 // physical cell mirrored by extended cell (t, cx, cy, cz): the image's periodic neighbour
-// (buffer_grid.f90:22-40), or the tile's own periodic image for independent periodic tiles
-__device__ __forceinline__ int32_t mirrored_cell(const DriftK &p, int t, int cx, int cy, int cz) {
-  const int c[3] = {cx, cy, cz};
-  const int tt[3] = {t % p.nnt, (t / p.nnt) % p.nnt, t / (p.nnt * p.nnt)};
-  int g[3];
+// (buffer_grid.f90:22-40), or the tile's own periodic image for independent periodic tiles; as tile
+// and local coordinates
+__device__ __forceinline__ void mirrored_cell(const DriftK &p, int t, int cx, int cy, int cz, int tt[3], int l[3]) {
+  const int ty = t / p.nnt, tz = ty / p.nnt;
+  tt[0] = t - ty * p.nnt;
+  tt[1] = ty - tz * p.nnt;
+  tt[2] = tz;
+  l[0] = cx - p.ncb;
+  l[1] = cy - p.ncb;
+  l[2] = cz - p.ncb;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    int l = c[d] - p.ncb;
-    if (p.tile_periodic) {
-      l = ((l % p.nt) + p.nt) % p.nt;
-      g[d] = tt[d] * p.nt + l;
-    } else {
-      const int x = tt[d] * p.nt + l;
-      g[d] = ((x % p.nc) + p.nc) % p.nc;
+    int w = 0;
+    while (l[d] < 0) l[d] += p.nt, w--;
+    while (l[d] >= p.nt) l[d] -= p.nt, w++;
+    if (!p.tile_periodic) {
+      tt[d] += w;
+      while (tt[d] < 0) tt[d] += p.nnt;
+      while (tt[d] >= p.nnt) tt[d] -= p.nnt;
     }
   }
-  return (g[2] * p.nc + g[1]) * p.nc + g[0];
 }
 
 // extended cell index of a physical cell in the tile that owns it
+__device__ __forceinline__ int64_t ext_cell(const DriftK &p, const int tt[3], const int l[3]) {
+  const int t = (tt[2] * p.nnt + tt[1]) * p.nnt + tt[0];
+  return (((int64_t)t * p.nte + l[2] + p.ncb) * p.nte + l[1] + p.ncb) * p.nte + l[0] + p.ncb;
+}
 __device__ __forceinline__ int64_t owner_ext_cell(const DriftK &p, int32_t G) {
-  const int gx = G % p.nc, gy = (G / p.nc) % p.nc, gz = G / (p.nc * p.nc);
-  const int t = ((gz / p.nt) * p.nnt + gy / p.nt) * p.nnt + gx / p.nt;
-  const int lx = gx % p.nt + p.ncb, ly = gy % p.nt + p.ncb, lz = gz % p.nt + p.ncb;
-  return (int64_t)t * p.nte * p.nte * p.nte + ((int64_t)lz * p.nte + ly) * p.nte + lx;
+  const int gy = G / p.nc, gz = gy / p.nc, g[3] = {G - gy * p.nc, gy - gz * p.nc, gz};
+  int tt[3], l[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    tt[d] = g[d] / p.nt;
+    l[d] = g[d] - tt[d] * p.nt;
+  }
+  return ext_cell(p, tt, l);
 }
 
 __global__ void k_ext_counts(DriftK p, const int32_t *phys_count, int32_t *rhoc_new) {
   const int64_t E = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (E >= p.ncells_src) return;
-  int t, cx, cy, cz;
+  int t, cx, cy, cz, tt[3], l[3];
   cell_of(p, E, t, cx, cy, cz);
-  rhoc_new[E] = phys_count[mirrored_cell(p, t, cx, cy, cz)];
+  mirrored_cell(p, t, cx, cy, cz, tt, l);
+  rhoc_new[E] = phys_count[((tt[2] * p.nt + l[2]) * p.nc + tt[1] * p.nt + l[1]) * p.nc + tt[0] * p.nt + l[0]];
 }
 
 __global__ void k_row_sums(const int32_t *rhoc, int64_t nrows, int nte, int64_t *rows) {
@@ -307,6 +367,21 @@ __global__ void __launch_bounds__(kDriftWarps * 32) k_runs_order(DriftK p) {
     const int s0 = p.dest_start[D], m = p.dest_start[D + 1] - s0;
     if (m == 0) continue;
     const int64_t start = p.cell_base_new[owner_ext_cell(p, (int32_t)D)];
+    if (m <= 32) {  // one run a lane, its key and count passed round by shuffles
+      const int32_t r = lane < m ? p.run_list[s0 + lane] : 0;
+      DriftRun o;
+      o.key = ~0ull;
+      o.count = 0;
+      if (lane < m) o = p.runs[r];
+      int off = 0;
+      for (int j = 0; j < m; j++) {
+        const uint64_t kj = __shfl_sync(0xffffffffu, o.key, j);
+        const int cj = __shfl_sync(0xffffffffu, o.count, j);
+        off += kj < o.key ? cj : 0;
+      }
+      if (lane < m) p.run_off[r] = start + off;
+      continue;
+    }
     for (int i = lane; i < m; i += 32) {
       const int32_t r = p.run_list[s0 + i];
       const uint64_t key = p.runs[r].key;
@@ -322,12 +397,14 @@ __global__ void __launch_bounds__(kDriftWarps * 32) k_runs_order(DriftK p) {
 
 // drift.f90:111: xp + nint(dt_mid*vp / (x_resolution*ratio_cs)), stored in int16 (wraps)
 __device__ __forceinline__ int16_t drift_offset(const DriftK &p, int16_t x, float v, int32_t *err) {
-  const double q = __ddiv_rn((double)__fmul_rn(p.dt_mid, v), p.xres_rcs);
+  const double dv = (double)__fmul_rn(p.dt_mid, v);
+  const double q = p.inv_rcs != 0.f ? __dmul_rn(dv, p.inv_xres_rcs) : __ddiv_rn(dv, p.xres_rcs);
   if (!(fabs(q) < 2147483647.0)) {  // nint beyond the default integer: undefined in the reference
     atomicOr(err, 1 << CUBE_ERR_INVALID);
     return x;
   }
-  const long long n = llround(q);
+  // nint: half away from zero.  The product form has at most 24 bits, so q +- 0.5 is exact
+  const int n = p.inv_rcs != 0.f ? __double2int_rz(q + copysign(0.5, q)) : (int)llround(q);
   return (int16_t)(uint16_t)((uint32_t)(int32_t)x + (uint32_t)n);
 }
 
@@ -385,19 +462,17 @@ __global__ void __launch_bounds__(kDriftWarps * 32) k_halo_fill(DriftK p, const 
     const int n = rhoc[E];
     if (n <= 0) continue;
     const int64_t dst = cell_base[E];
-    const int64_t src = cell_base[owner_ext_cell(p, mirrored_cell(p, t, cx, cy, cz))];
+    int tt[3], l[3];
+    mirrored_cell(p, t, cx, cy, cz, tt, l);
+    const int64_t src = cell_base[ext_cell(p, tt, l)];
     if (dst < 0 || src < 0 || dst + n > p.n_used_new || src + n > p.n_used_new) continue;  // inconsistent spine
-    for (int l = lane; l < n; l += 32) {
-      if (xp) {
-        xp[3 * (dst + l) + 0] = xp[3 * (src + l) + 0];
-        xp[3 * (dst + l) + 1] = xp[3 * (src + l) + 1];
-        xp[3 * (dst + l) + 2] = xp[3 * (src + l) + 2];
-      }
-      vp[3 * (dst + l) + 0] = vp[3 * (src + l) + 0];
-      vp[3 * (dst + l) + 1] = vp[3 * (src + l) + 1];
-      vp[3 * (dst + l) + 2] = vp[3 * (src + l) + 2];
-      if (pid) pid[dst + l] = pid[src + l];
+    // the cell's arrays are contiguous on both sides: copied value by value, coalesced
+    for (int i = lane; i < 3 * n; i += 32) {
+      if (xp) xp[3 * dst + i] = xp[3 * src + i];
+      vp[3 * dst + i] = vp[3 * src + i];
     }
+    if (pid)
+      for (int i = lane; i < n; i += 32) pid[dst + i] = pid[src + i];
   }
 }
 
@@ -417,6 +492,8 @@ static DriftK make_driftk(const DriftArgs &a) {
   p.dt_mid = a.dt_mid;
   p.rcs_f = (float)L.rcs;
   p.xres_rcs = (1.0 / 65536.0) * (double)L.rcs;
+  p.inv_rcs = (L.rcs & (L.rcs - 1)) ? 0.f : 1.0f / (float)L.rcs;
+  p.inv_xres_rcs = 1.0 / p.xres_rcs;
   p.rhoc = a.rhoc;
   p.cell_base = a.cell_base;
   p.xp = a.xp;
