@@ -92,7 +92,7 @@ struct Ctx {
   Buf xp, rhoc, idx, vp, cell_base;
   Buf tiles, count, cell_start, scan_tmp, spos, spill, spill_rank, counters, items, range_loc, sched;
   Buf rho, rhok, force, jobs, out;
-  Buf mlp_pos, mlp_rho;  // learned shell: positions of the stored copies, fine-grid CIC density
+  Buf mlp_pos, mlp_rho, mlp_n;  // learned shell: positions of the copies, fine-grid CIC density, listed copies
   // PP kernel shape: fixed (pp_fixed >= 0, cube_pp_set_shape) or autotuned, keyed by
   // pp_shape_key; pp_ms holds the last tuning's times, pp_last the shape of the last PP kick
   int pp_fixed = -1;
@@ -522,21 +522,9 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     CK(grow(g.rho, sizeof(float) * n3 * nslots));
     CK(grow(g.rhok, sizeof(cufftComplex) * nk * nslots));
     const double scale = (double)L.rcs / (double)(1.0f / (float)rsf);
-    std::vector<MeshJob> jobs(L.ntile);
-    for (int t = 0; t < L.ntile; t++) {
-      const int tx = t % L.nnt, ty = (t / L.nnt) % L.nnt, tz = t / (L.nnt * L.nnt);
-      MeshJob &J = jobs[t];
-      J.t = t;
-      J.slot = per_tile ? t : 0;
-      J.range = 0.f;
-      const int tc[3] = {tx, ty, tz};
-      for (int q = 0; q < 3; q++) {
-        J.lo[q] = L.ncb;
-        J.alo[q] = L.ncb;
-        J.off[q] = per_tile ? 0.0 : -(double)tc[q] * L.nt * scale;
-      }
-    }
-    CK(upload(g.jobs, jobs.data(), jobs.size(), soff));
+    CK(grow(g.jobs, sizeof(MeshJob) * (size_t)L.ntile));
+    launch_mesh_jobs(L, scale, per_tile, (MeshJob *)g.jobs.p, g.stream);
+    g.launches += 1;
     PM3Args a{};
     a.L = &g.L;
     a.rsf = rsf;
@@ -1947,21 +1935,64 @@ int cube_mlp_get_params(cube_mlp *h, float *params, float *grads) {
   return CUBE_OK;
 }
 
-// positions of the stored copies and the fine-grid density of the image, on stream s
-static int mlp_prepare(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const int16_t *d_xp, int64_t n_used,
-                       cudaStream_t s) {
+// log(1 + density) on the fine grid of the image, on g.stream.  With `list`, the interior copies are listed in
+// g.mlp_pos (g.mlp_n of them).
+static int mlp_density(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const int16_t *d_xp, int64_t n_used, bool list) {
   const Lay &L = g.L;
   if (L.pm3_mode != CUBE_PM3_PERIODIC) return fail(CUBE_ERR_INVALID);  // one periodic image
+  cudaStream_t s = g.stream;
+  const int64_t ng3 = (int64_t)L.ng * L.ng * L.ng;
   CK(grow(g.cell_base, sizeof(int64_t) * (size_t)L.ntile * L.nte * L.nte * L.nte));
   CK(grow(g.mlp_pos, sizeof(float4) * (size_t)std::max<int64_t>(n_used, 1)));
-  CK(grow(g.mlp_rho, sizeof(float) * (size_t)L.ng * L.ng * L.ng));
+  CK(grow(g.mlp_rho, sizeof(float) * (size_t)ng3));
+  CK(grow(g.mlp_n, sizeof(unsigned long long)));
+  CK(grow(g.jobs, sizeof(MeshJob) * (size_t)L.ntile));
+  launch_mesh_jobs(L, (double)L.rcs, false, (MeshJob *)g.jobs.p, s);
   launch_cell_table(L, d_rhoc, d_idx_b_r, (int64_t *)g.cell_base.p, s);
-  launch_mlp_pos(L, d_xp, d_rhoc, (const int64_t *)g.cell_base.p, (float4 *)g.mlp_pos.p, s);
-  launch_mlp_density((const float4 *)g.mlp_pos.p, n_used, L.ng, (float *)g.mlp_rho.p, s);
+  CU(cudaMemsetAsync(g.mlp_rho.p, 0, sizeof(float) * ng3, s));
+  PM3Args a{};  // the fine grid as a mesh of ratio_cs points per coarse cell
+  a.L = &g.L;
+  a.n = L.ng;
+  a.nslots = 1;
+  a.jobs = (const MeshJob *)g.jobs.p;
+  a.njobs = L.ntile;
+  for (int q = 0; q < 3; q++) a.rdep[q] = a.ract[q] = L.nt;
+  a.wrap = 1;
+  a.scale = (double)L.rcs;
+  a.xp = d_xp;
+  a.rhoc = d_rhoc;
+  a.cell_base = (const int64_t *)g.cell_base.p;
+  a.rho = (float *)g.mlp_rho.p;
+  a.num_sms = g.num_sms;
+  CK(grow(g.dep_items, pm3_dep_items_bytes((int64_t)L.nt * L.nt * L.nt, L.ntile, n_used)));
+  a.dep_items = (int2 *)g.dep_items.p;
+  a.n_particles_hint = n_used;
+  const bool bricks = pm3_brick_mc(a) > 0;
+  if (list || !bricks) {
+    launch_mlp_list(L, d_xp, d_rhoc, (const int64_t *)g.cell_base.p, (float4 *)g.mlp_pos.p,
+                    (unsigned long long *)g.mlp_n.p, s);
+    g.launches += 1;
+  }
+  if (bricks) {
+    g.launches += launch_cic_bricks(a, s);
+  } else {
+    launch_mlp_cic((const float4 *)g.mlp_pos.p, (const unsigned long long *)g.mlp_n.p, L.ng, (float *)g.mlp_rho.p, s);
+    g.launches += 1;
+  }
+  launch_mlp_log1p((float *)g.mlp_rho.p, ng3, s);
   g.launches += 3;
   CU(cudaGetLastError());
   return CUBE_OK;
 }
+
+// the library's stream is the caller's while an entry point runs
+struct StreamScope {
+  cudaStream_t own;
+  explicit StreamScope(void *s) : own(g.stream) {
+    if (s) g.stream = (cudaStream_t)s;
+  }
+  ~StreamScope() { g.stream = own; }
+};
 
 int cube_mlp_features(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const int16_t *d_xp, int64_t n_used,
                       void *d_X, void *stream) {
@@ -1970,8 +2001,11 @@ int cube_mlp_features(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const int
   if (!g.configured) return fail(CUBE_ERR_NOT_CONFIGURED);
   if (!d_rhoc || !d_idx_b_r || !d_xp || !d_X || n_used < 0) return fail(CUBE_ERR_INVALID);
   CK(ensure_device());
-  cudaStream_t s = stream ? (cudaStream_t)stream : g.stream;
-  CK(mlp_prepare(d_rhoc, d_idx_b_r, d_xp, n_used, s));
+  const StreamScope scope(stream);
+  cudaStream_t s = g.stream;
+  CK(mlp_density(d_rhoc, d_idx_b_r, d_xp, n_used, false));
+  launch_mlp_pos(g.L, d_xp, d_rhoc, (const int64_t *)g.cell_base.p, (float4 *)g.mlp_pos.p, s);
+  g.launches += 1;
   launch_mlp_features((const float4 *)g.mlp_pos.p, n_used, (const float *)g.mlp_rho.p, g.L.ng,
                       (__nv_bfloat16 *)d_X, s);
   g.launches += 1;
@@ -2006,12 +2040,13 @@ int cube_mlp_kick(cube_mlp *h, const int32_t *d_rhoc, const int64_t *d_idx_b_r, 
   if (!g.configured) return fail(CUBE_ERR_NOT_CONFIGURED);
   if (!h || !d_rhoc || !d_idx_b_r || !d_xp || !d_vp || n_used < 0) return fail(CUBE_ERR_INVALID);
   CK(ensure_device());
-  cudaStream_t s = stream ? (cudaStream_t)stream : g.stream;
-  CK(mlp_prepare(d_rhoc, d_idx_b_r, d_xp, n_used, s));
+  const StreamScope scope(stream);
+  cudaStream_t s = g.stream;
+  CK(mlp_density(d_rhoc, d_idx_b_r, d_xp, n_used, true));
   // the kick coefficient of run_kick (kick.f90:529), times the network's output scale
   const float kick = (float)((double)(a_mid * dt / 6.0f) / 3.14159265358979323846);
-  launch_mlp_apply(h->p, (const float4 *)g.mlp_pos.p, (const float *)g.mlp_rho.p, g.L.ng, n_used, d_vp,
-                   kick * scale, g.num_sms, s);
+  launch_mlp_apply(h->p, (const float4 *)g.mlp_pos.p, (const unsigned long long *)g.mlp_n.p,
+                   (const float *)g.mlp_rho.p, g.L.ng, d_vp, kick * scale, g.num_sms, s);
   g.launches += 1;
   CU(cudaGetLastError());
   // the inference kernel's bounded waits report through a status word: read it once the kick is done
@@ -2167,6 +2202,7 @@ void c_pm3_fft_finalize(void) {
   release(g.jobs);
   release(g.mlp_pos);
   release(g.mlp_rho);
+  release(g.mlp_n);
 }
 
 void c_gpu_velocity_finalize(void) {

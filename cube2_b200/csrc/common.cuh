@@ -262,7 +262,11 @@ struct PM3Args {
 // scratch of the deposit work list for a launch over `njobs` jobs of `cells` coarse cells each
 size_t pm3_dep_items_bytes(int64_t cells_per_job, int njobs, int64_t n_used);
 constexpr int kPotPad = 4;  // ghost points per side of the padded potential of the brick kernels
+// mesh jobs of the periodic geometries: one mesh over the image, or one per tile
+void launch_mesh_jobs(const Lay &L, double scale, bool per_tile, MeshJob *jobs, cudaStream_t s);
 int launch_pm3_deposit(const PM3Args &a, cudaStream_t s);  // returns the kernels it launched
+// CIC instead of TSC on the brick kernels' geometry (pm3_brick_mc != 0, else nothing and 0): cell-centred points
+int launch_cic_bricks(const PM3Args &a, cudaStream_t s);
 void launch_pm3_kspace(const PM3Args &a, cudaStream_t s);
 // the k-space step on the spectrum of two-dimensional x-y transforms: z transform, Green
 // multiply, inverse z transform (mesh sides where pm3_kspace_z_ok)
@@ -380,10 +384,14 @@ struct MlpParams {
 };
 void launch_mlp_pos(const Lay &L, const int16_t *xp, const int32_t *rhoc, const int64_t *cell_base, float4 *pos,
                     cudaStream_t s);
-void launch_mlp_density(const float4 *pos, int64_t n, int ng, float *rho, cudaStream_t s);
+// the interior copies as a list (fine position, w = storage index) and their number
+void launch_mlp_list(const Lay &L, const int16_t *xp, const int32_t *rhoc, const int64_t *cell_base, float4 *list,
+                     unsigned long long *n_list, cudaStream_t s);
+void launch_mlp_cic(const float4 *list, const unsigned long long *n_list, int ng, float *rho, cudaStream_t s);
+void launch_mlp_log1p(float *rho, int64_t n, cudaStream_t s);
 void launch_mlp_features(const float4 *pos, int64_t n, const float *rho, int ng, __nv_bfloat16 *X, cudaStream_t s);
-void launch_mlp_apply(const MlpParams &m, const float4 *pos, const float *rho, int ng, int64_t n, float *vp,
-                      float coef, int num_sms, cudaStream_t s);
+void launch_mlp_apply(const MlpParams &m, const float4 *list, const unsigned long long *n_list, const float *rho, int ng,
+                      float *vp, float coef, int num_sms, cudaStream_t s);
 void launch_mlp_pack(MlpParams &m, cudaStream_t s);
 int mlp_train_step(MlpParams &m, const __nv_bfloat16 *X, const float *T, const int32_t *rows, int batch, float lr,
                    float *loss, cudaStream_t s);

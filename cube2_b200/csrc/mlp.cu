@@ -66,13 +66,75 @@ __global__ void __launch_bounds__(kWarps * 32) k_mlp_pos(MlpPosK p) {
   }
 }
 
+// The interior copies alone, as a list: a block takes 32 physical coarse cells, reserves their places with
+// one atomic and writes fine position and storage index (w).  The order of the list does not matter to
+// the kick (every particle's output depends on its own inputs only).  The position is the one of
+// k_mlp_pos: c ratio_cs and (2u + 1) ratio_cs / 2^17 are exact in FP32, so their sum rounds once.
+constexpr int kListCells = 32;
+struct MlpListK {
+  int nt, nte, ncb, nnt, rcs, ng;
+  int64_t ncells;  // physical coarse cells of the image
+  const int16_t *xp;
+  const int32_t *rhoc;
+  const int64_t *cell_base;
+  float4 *list;
+  unsigned long long *n_list;  // zeroed
+};
+__global__ void __launch_bounds__(kWarps * 32) k_mlp_list(MlpListK p) {
+  __shared__ int s_n[kListCells], s_off[kListCells], s_c[3][kListCells];
+  __shared__ int64_t s_base[kListCells];
+  __shared__ unsigned long long s_first;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) {  // lane = cell
+    const int64_t c = (int64_t)blockIdx.x * kListCells + lane;
+    int np = 0;
+    if (c < p.ncells) {
+      const unsigned nt = (unsigned)p.nt, u = (unsigned)c, q = u / nt, qq = q / nt, t = qq / nt;
+      const int i = (int)(u - q * nt), j = (int)(q - qq * nt), k = (int)(qq - t * nt);
+      const int tx = (int)t % p.nnt, ty = (int)t / p.nnt % p.nnt, tz = (int)t / (p.nnt * p.nnt);
+      const int64_t e = (((int64_t)t * p.nte + k + p.ncb) * p.nte + j + p.ncb) * p.nte + i + p.ncb;
+      np = p.rhoc[e];
+      s_base[lane] = p.cell_base[e];
+      s_c[0][lane] = tx * p.nt + i;
+      s_c[1][lane] = ty * p.nt + j;
+      s_c[2][lane] = tz * p.nt + k;
+    }
+    int incl = np;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    s_n[lane] = np;
+    s_off[lane] = incl - np;
+    if (lane == 31) s_first = atomicAdd(p.n_list, (unsigned long long)incl);
+  }
+  __syncthreads();
+  const float ulp = (float)p.rcs * (1.0f / 131072.0f);
+  for (int cc = warp; cc < kListCells; cc += kWarps) {
+    const int np = s_n[cc];
+    float4 *dst = p.list + s_first + s_off[cc];
+    const int64_t base = s_base[cc];
+    const float c0 = (float)(s_c[0][cc] * p.rcs), c1 = (float)(s_c[1][cc] * p.rcs), c2 = (float)(s_c[2][cc] * p.rcs);
+    for (int l = lane; l < np; l += 32) {
+      const int16_t *q = p.xp + 3 * (base + l);
+      float v[3] = {c0 + (float)(2 * (int)(uint16_t)q[0] + 1) * ulp, c1 + (float)(2 * (int)(uint16_t)q[1] + 1) * ulp,
+                    c2 + (float)(2 * (int)(uint16_t)q[2] + 1) * ulp};
+#pragma unroll
+      for (int d = 0; d < 3; d++)
+        if (v[d] >= (float)p.ng) v[d] = 0.f;
+      dst[l] = make_float4(v[0], v[1], v[2], __int_as_float((int)(base + l)));
+    }
+  }
+}
+
 __device__ __forceinline__ int wrap_cell(int i, int ng) { return i < 0 ? i + ng : (i >= ng ? i - ng : i); }
 
-// CIC density of the interior copies (each physical particle once) on the periodic fine grid
-__global__ void k_mlp_cic(const float4 *pos, int64_t n, int ng, float *rho) {
+// CIC density of the listed copies (each physical particle once) on the periodic fine grid, by float atomics:
+// for layouts that the brick deposit does not take
+__global__ void k_mlp_cic(const float4 *list, const unsigned long long *n_list, int ng, float *rho) {
+  const int64_t n = (int64_t)*n_list;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float4 q = pos[i];
-    if (q.w == 0.f) continue;
+    const float4 q = list[i];
     const float xs[3] = {q.x - 0.5f, q.y - 0.5f, q.z - 0.5f};
     int i0[3];
     float f[3];
@@ -168,6 +230,15 @@ __device__ __forceinline__ float gelu_f(float z) {
   const float t = tanh_hw(gelu_tanh_arg(z));
   const float hz = 0.5f * z;
   return fmaf(hz, t, hz);
+}
+
+// two of them on f32x2 arithmetic, every operation rounded as its scalar form
+__device__ __forceinline__ float2 gelu2(float2 z) {
+  const float2 c = make_float2(kGeluC, kGeluC), c3 = make_float2(kGeluC3, kGeluC3);
+  const float2 u = __fmul2_rn(z, __ffma2_rn(c3, __fmul2_rn(z, z), c));
+  const float2 t = make_float2(tanh_hw(u.x), tanh_hw(u.y));
+  const float2 hz = __fmul2_rn(make_float2(0.5f, 0.5f), z);
+  return __ffma2_rn(hz, t, hz);
 }
 
 __device__ __forceinline__ float gelu_grad_f(float z) {
@@ -353,10 +424,10 @@ constexpr size_t kApplySmem = sizeof(bf16) * ((size_t)kMlpW * kLd1 + 2 * (size_t
 struct MlpApplyK {
   const bf16 *wb;
   const float *master;
-  const float4 *pos;
+  const float4 *list;  // interior copies: fine position, w = storage index
+  const unsigned long long *n_list;
   const float *rho;
   int ng;
-  int64_t n;
   float *vp;
   float coef;  // kick coefficient times the output scale
 };
@@ -426,7 +497,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, 1) k_mlp_apply(MlpApplyK p) 
   __syncthreads();
 
   const int g = lane >> 2, t = lane & 3;
-  const int64_t ntiles = (p.n + 15) / 16;
+  const int64_t n = (int64_t)*p.n_list, ntiles = (n + 15) / 16;
   for (int64_t tile = (int64_t)blockIdx.x * kApplyWarps + warp; tile < ntiles;
        tile += (int64_t)gridDim.x * kApplyWarps) {
     const int64_t r0 = tile * 16;
@@ -435,9 +506,8 @@ __global__ void __launch_bounds__(kApplyWarps * 32, 1) k_mlp_apply(MlpApplyK p) 
       const int rr = lane >> 1, half = lane & 1;
       const int64_t i = r0 + rr;
       __align__(16) bf16 row[kMlpK1];
-      const float4 q = i < p.n ? p.pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (i < p.n && q.w != 0.f) {
-        mlp_inputs(q, p.rho, p.ng, row);
+      if (i < n) {
+        mlp_inputs(p.list[i], p.rho, p.ng, row);
       } else {
         for (int j = 0; j < kMlpK1; j++) row[j] = __float2bfloat16_rn(0.f);
       }
@@ -462,8 +532,8 @@ __global__ void __launch_bounds__(kApplyWarps * 32, 1) k_mlp_apply(MlpApplyK p) 
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int64_t i = r0 + g + 8 * h;
-        if (i >= p.n || p.pos[i].w == 0.f) continue;
-        float *v = p.vp + 3 * i + 2 * t;
+        if (i >= n) continue;
+        float *v = p.vp + 3 * (int64_t)__float_as_int(p.list[i].w) + 2 * t;
         v[0] += p.coef * (acc[2 * h] + bias[3 * kMlpW + 2 * t]);
         if (t == 0) v[1] += p.coef * (acc[2 * h + 1] + bias[3 * kMlpW + 1]);
       }
@@ -647,8 +717,8 @@ __device__ __forceinline__ void tc_inputs(float4 q, bool live, const float *__re
   int X[4];
 #pragma unroll
   for (int dx = 0; dx < 4; dx++) X[dx] = wrap_cell(i0[0] + dx - 1, ng);
-#pragma unroll 1
-  for (int c = 0; c < 8; c++) {
+#pragma unroll 4
+  for (int c = 0; c < 8; c++) {  // 32 loads in flight
     const int dz = c >> 1, h = c & 1;
     const int64_t Z = wrap_cell(wrap_cell(i0[2] + dz - 1, ng), ng);
     __align__(16) __nv_bfloat162 v[4];
@@ -730,12 +800,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_apply_tc(MlpApplyK p, int
   uint32_t phase = 0;
   bool ok = true;
 
-  const int64_t ntiles = (p.n + kTcRows - 1) / kTcRows;
+  const int64_t n = (int64_t)*p.n_list, ntiles = (n + kTcRows - 1) / kTcRows;
   for (int64_t tile = (int64_t)blockIdx.x * kTcGroups + wg; tile < ntiles && ok;
        tile += (int64_t)gridDim.x * kTcGroups) {
     const int64_t i = tile * kTcRows + m;
-    const float4 q = i < p.n ? p.pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const bool live = i < p.n && q.w != 0.f;
+    const bool live = i < n;
+    const float4 q = live ? p.list[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     tc_inputs(q, live, p.rho, p.ng, act, m);  // layer-1 input row of this particle
     // layers 1-3 (N = 128): MMA, then bias + GELU + BF16 back into the activation buffer
 #pragma unroll 1
@@ -758,8 +828,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_apply_tc(MlpApplyK p, int
         tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
         __align__(16) __nv_bfloat162 h[8];
 #pragma unroll
-        for (int j = 0; j < 8; j++)
-          h[j] = __floats2bfloat162_rn(gelu_f(v[2 * j] + b[c0 + 2 * j]), gelu_f(v[2 * j + 1] + b[c0 + 2 * j + 1]));
+        for (int j = 0; j < 8; j++) {
+          const float2 b2 = *reinterpret_cast<const float2 *>(b + c0 + 2 * j);
+          const float2 a = gelu2(__fadd2_rn(make_float2(v[2 * j], v[2 * j + 1]), b2));
+          h[j] = __floats2bfloat162_rn(a.x, a.y);
+        }
 #pragma unroll
         for (int c = 0; c < 2; c++)
           *reinterpret_cast<uint4 *>(act + umma_off(m, c0 + 8 * c, kTcRows)) = reinterpret_cast<const uint4 *>(h)[c];
@@ -781,7 +854,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_apply_tc(MlpApplyK p, int
     float y[4];
     tmem_ld4(tmem + lane_base, y);
     if (live) {
-      float *v = p.vp + 3 * i;
+      float *v = p.vp + 3 * (int64_t)__float_as_int(q.w);
       v[0] += p.coef * (y[0] + bias[3 * kMlpW + 0]);
       v[1] += p.coef * (y[1] + bias[3 * kMlpW + 1]);
       v[2] += p.coef * (y[2] + bias[3 * kMlpW + 2]);
@@ -1252,11 +1325,18 @@ __global__ void k_mlp_log1p(float *rho, int64_t n) {
     rho[i] = log1pf(rho[i]);
 }
 
-void launch_mlp_density(const float4 *pos, int64_t n, int ng, float *rho, cudaStream_t s) {
-  cudaMemsetAsync(rho, 0, sizeof(float) * (size_t)ng * ng * ng, s);
-  k_mlp_cic<<<148 * 8, 256, 0, s>>>(pos, n, ng, rho);
-  k_mlp_log1p<<<148 * 8, 256, 0, s>>>(rho, (int64_t)ng * ng * ng);
+void launch_mlp_list(const Lay &L, const int16_t *xp, const int32_t *rhoc, const int64_t *cell_base, float4 *list,
+                     unsigned long long *n_list, cudaStream_t s) {
+  cudaMemsetAsync(n_list, 0, sizeof(unsigned long long), s);
+  MlpListK p{L.nt, L.nte, L.ncb, L.nnt, L.rcs, L.ng, (int64_t)L.ntile * L.nt * L.nt * L.nt, xp, rhoc, cell_base, list, n_list};
+  k_mlp_list<<<(unsigned)((p.ncells + kListCells - 1) / kListCells), kWarps * 32, 0, s>>>(p);
 }
+
+void launch_mlp_cic(const float4 *list, const unsigned long long *n_list, int ng, float *rho, cudaStream_t s) {
+  k_mlp_cic<<<148 * 8, 256, 0, s>>>(list, n_list, ng, rho);
+}
+
+void launch_mlp_log1p(float *rho, int64_t n, cudaStream_t s) { k_mlp_log1p<<<148 * 8, 256, 0, s>>>(rho, n); }
 
 void launch_mlp_features(const float4 *pos, int64_t n, const float *rho, int ng, bf16 *X, cudaStream_t s) {
   k_mlp_features<<<148 * 8, 256, 0, s>>>(pos, n, rho, ng, X);
@@ -1284,15 +1364,15 @@ void launch_gemm_nt(const bf16 *A, int lda, const bf16 *B, int ldb, int M, int N
   k_gemm_nt<<<grid, 128, 0, s>>>(A, lda, B, ldb, M, N, K, bias, Z, ldz, H, ldh, act);
 }
 
-void launch_mlp_apply(const MlpParams &m, const float4 *pos, const float *rho, int ng, int64_t n, float *vp,
-                      float coef, int num_sms, cudaStream_t s) {
+void launch_mlp_apply(const MlpParams &m, const float4 *list, const unsigned long long *n_list, const float *rho, int ng,
+                      float *vp, float coef, int num_sms, cudaStream_t s) {
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(k_mlp_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kApplySmem);
     cudaFuncSetAttribute(k_mlp_apply_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
     attr = true;
   }
-  MlpApplyK p{m.wb, m.master, pos, rho, ng, n, vp, coef};
+  MlpApplyK p{m.wb, m.master, list, n_list, rho, ng, vp, coef};
   if (getenv("CUBE_MLP_MMA_SYNC")) {
     k_mlp_apply<<<num_sms, kApplyWarps * 32, kApplySmem, s>>>(p);
   } else {

@@ -77,6 +77,13 @@ __device__ __forceinline__ int tsc_brick(int d, int16_t xp, int mc, float w[3]) 
   return d * mc + (int)(q >> 17);
 }
 
+// the same for CIC on cell-centred points: floor(x - 1/2) and its fraction
+__device__ __forceinline__ int cic_brick(int d, int16_t xp, int mc, float &f) {
+  const int q = (int)((2u * (uint16_t)xp + 1u) * (unsigned)mc) - 65536;
+  f = (float)(q & 0x1ffff) * (1.0f / 131072.0f);
+  return d * mc + (q >> 17);
+}
+
 __global__ void __launch_bounds__(kWarps * 32) k_deposit(PM3K p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t cells = (int64_t)p.rdep[0] * p.rdep[1] * p.rdep[2];
@@ -1122,6 +1129,7 @@ __global__ void k_dep_items(PM3K p, int mc, int64_t nbricks, int chunk, int2 *it
   }
 }
 
+template <bool CIC>
 __global__ void __launch_bounds__(kDepThreads, kDepBlocks) k_deposit_brick(PM3K p, int mc, const int2 *items,
                                                                                const int *count, int cap) {
   __shared__ __align__(16) unsigned acc[kAccW * kAccW * kAccX];
@@ -1146,14 +1154,29 @@ __global__ void __launch_bounds__(kDepThreads, kDepBlocks) k_deposit_brick(PM3K 
       __syncthreads();
       continue;
     }
-    // fixed-point scale 2^e: particles * 0.4219 * 2^e < 2^32
+    // fixed-point scale 2^e: particles * (largest weight) * 2^e < 2^32
     int e = 24;
-    while (e > 1 && (double)(k1 - k0) * 0.421875 * (double)(1u << e) >= 4294967040.0) e--;
+    while (e > 1 && (double)(k1 - k0) * (CIC ? 1.0 : 0.421875) * (double)(1u << e) >= 4294967040.0) e--;
     const float fs = (float)(1u << e), inv = 1.0f / fs;
     for (int k = k0 + threadIdx.x; k < k1; k += kDepThreads) {
       int di, dj, dk;
       const int64_t ip = brick_particle(k, br, rbase, rstart, rcell, di, dj, dk);
       const int16_t *qp = p.xp + 3 * ip;
+      if constexpr (CIC) {  // points at cell centres: the first is floor(x - 1/2), from -1 of the brick on
+        float fx, fy, fz;
+        const int lx = cic_brick(di, qp[0], mc, fx) + 4, ly = cic_brick(dj, qp[1], mc, fy) + 1,
+                  lz = cic_brick(dk, qp[2], mc, fz) + 1;
+        const float sx[2] = {(1.0f - fx) * fs, fx * fs}, sy[2] = {1.0f - fy, fy}, sz[2] = {1.0f - fz, fz};
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+#pragma unroll
+          for (int bb = 0; bb < 2; bb++) {
+            unsigned *row = acc + ((lz + c) * kAccW + (ly + bb)) * kAccX + lx;
+            atomicAdd(row + 0, __float2uint_rn(sx[0] * sy[bb] * sz[c]));
+            atomicAdd(row + 1, __float2uint_rn(sx[1] * sy[bb] * sz[c]));
+          }
+        continue;
+      }
       float wx[3], wy[3], wz[3];
       // window indices of the stencil's first point: x (ix - 1) - (X0 - 4), y (iy - 1) - (Y0 - 1)
       const int lx = tsc_brick(di, qp[0], mc, wx) + 3, ly = tsc_brick(dj, qp[1], mc, wy), lz = tsc_brick(dk, qp[2], mc, wz);
@@ -1230,32 +1253,59 @@ size_t pm3_dep_items_bytes(int64_t cells_per_job, int njobs, int64_t n_used) {
   return sizeof(int2) * ((size_t)cells_per_job * njobs + (size_t)(n_used / kDepChunk) + 2);
 }
 
-int launch_pm3_deposit(const PM3Args &a, cudaStream_t s) {
-  PM3K p = make_k(a);
-  const int mc = pm3_brick_mc(a);
-  if (mc) {
-    constexpr int chunk = kDepChunk;
-    auto kern = k_deposit_brick;
-    const int cb = kBrick / mc;
-    const int64_t nbricks = (int64_t)bricks_of(a.rdep[0], cb) * bricks_of(a.rdep[1], cb) * bricks_of(a.rdep[2], cb) * a.njobs;
-    if (nbricks <= 0) return 0;
-    const int64_t resident = (int64_t)(a.num_sms > 0 ? a.num_sms : 148) * kDepBlocks;
-    if (!a.dep_items) {
-      kern<<<(unsigned)std::min(nbricks, resident), kDepThreads, 0, s>>>(p, mc, nullptr, nullptr, (int)nbricks);
-      return 1;
+// Mesh jobs of the periodic geometries, one per tile: written on the device, so that no host table has to cross
+// (and a captured call replays from nothing but device memory)
+__global__ void k_mesh_jobs(MeshJob *jobs, int ntile, int nnt, int nt, int ncb, double scale, int per_tile) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntile; t += gridDim.x * blockDim.x) {
+    const int tc[3] = {t % nnt, (t / nnt) % nnt, t / (nnt * nnt)};
+    MeshJob J;
+    J.t = t;
+    J.slot = per_tile ? t : 0;
+    J.range = 0.f;
+    for (int q = 0; q < 3; q++) {
+      J.lo[q] = J.alo[q] = ncb;
+      J.off[q] = per_tile ? 0.0 : -(double)tc[q] * nt * scale;
     }
-    // at most one item per brick plus one per `chunk` particles
-    const int64_t cap = nbricks + a.n_particles_hint / chunk + 1;
-    int *count = reinterpret_cast<int *>(a.dep_items + cap);
-    cudaMemsetAsync(count, 0, sizeof(int), s);
-    k_dep_items<<<(unsigned)std::min<int64_t>((nbricks + 255) / 256, 4096), 256, 0, s>>>(p, mc, nbricks, chunk,
-                                                                                       a.dep_items, count, cap);
-    kern<<<(unsigned)std::min(cap, resident), kDepThreads, 0, s>>>(p, mc, a.dep_items, count, (int)cap);
-    return 2;
+    jobs[t] = J;
   }
+}
+void launch_mesh_jobs(const Lay &L, double scale, bool per_tile, MeshJob *jobs, cudaStream_t s) {
+  k_mesh_jobs<<<(unsigned)std::min((L.ntile + 127) / 128, 148), 128, 0, s>>>(jobs, L.ntile, L.nnt, L.nt, L.ncb, scale, per_tile);
+}
+
+// the brick deposit (TSC or CIC), with its work list where the caller gives the scratch for one
+template <bool CIC>
+static int launch_deposit_bricks(const PM3Args &a, int mc, cudaStream_t s) {
+  const PM3K p = make_k(a);
+  const int cb = kBrick / mc;
+  const int64_t nbricks = (int64_t)bricks_of(a.rdep[0], cb) * bricks_of(a.rdep[1], cb) * bricks_of(a.rdep[2], cb) * a.njobs;
+  if (nbricks <= 0) return 0;
+  const int64_t resident = (int64_t)(a.num_sms > 0 ? a.num_sms : 148) * kDepBlocks;
+  if (!a.dep_items) {
+    k_deposit_brick<CIC><<<(unsigned)std::min(nbricks, resident), kDepThreads, 0, s>>>(p, mc, nullptr, nullptr, (int)nbricks);
+    return 1;
+  }
+  // at most one item per brick plus one per kDepChunk particles
+  const int64_t cap = nbricks + a.n_particles_hint / kDepChunk + 1;
+  int *count = reinterpret_cast<int *>(a.dep_items + cap);
+  cudaMemsetAsync(count, 0, sizeof(int), s);
+  k_dep_items<<<(unsigned)std::min<int64_t>((nbricks + 255) / 256, 4096), 256, 0, s>>>(p, mc, nbricks, kDepChunk,
+                                                                                     a.dep_items, count, cap);
+  k_deposit_brick<CIC><<<(unsigned)std::min(cap, resident), kDepThreads, 0, s>>>(p, mc, a.dep_items, count, (int)cap);
+  return 2;
+}
+
+int launch_pm3_deposit(const PM3Args &a, cudaStream_t s) {
+  if (const int mc = pm3_brick_mc(a)) return launch_deposit_bricks<false>(a, mc, s);
+  const PM3K p = make_k(a);
   const int64_t warps = (int64_t)a.rdep[0] * a.rdep[1] * a.rdep[2] * a.njobs;
   k_deposit<<<(unsigned)((warps + kWarps - 1) / kWarps), kWarps * 32, 0, s>>>(p);
   return 1;
+}
+
+int launch_cic_bricks(const PM3Args &a, cudaStream_t s) {
+  const int mc = pm3_brick_mc(a);
+  return mc ? launch_deposit_bricks<true>(a, mc, s) : 0;
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link to libcuda)
