@@ -358,39 +358,47 @@ __global__ void k_runs_fill(DriftK p, int32_t nruns) {
   p.run_list[p.dest_start[D] + slot] = r;
 }
 
-// warp per destination cell: first slot of each of its runs = the cell's start plus the
-// particles of its runs with a smaller visiting key
+// eight lanes per destination cell (it has few runs: its own and those of the neighbours that send copies): first
+// slot of each of its runs = the cell's start plus the particles of its runs with a smaller visiting key
 __global__ void __launch_bounds__(kDriftWarps * 32) k_runs_order(DriftK p) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t ndest = (int64_t)p.nc * p.nc * p.nc;
-  for (int64_t D = (int64_t)blockIdx.x * kDriftWarps + warp; D < ndest; D += (int64_t)gridDim.x * kDriftWarps) {
-    const int s0 = p.dest_start[D], m = p.dest_start[D + 1] - s0;
-    if (m == 0) continue;
-    const int64_t start = p.cell_base_new[owner_ext_cell(p, (int32_t)D)];
-    if (m <= 32) {  // one run a lane, its key and count passed round by shuffles
-      const int32_t r = lane < m ? p.run_list[s0 + lane] : 0;
-      DriftRun o;
-      o.key = ~0ull;
-      o.count = 0;
-      if (lane < m) o = p.runs[r];
-      int off = 0;
-      for (int j = 0; j < m; j++) {
-        const uint64_t kj = __shfl_sync(0xffffffffu, o.key, j);
-        const int cj = __shfl_sync(0xffffffffu, o.count, j);
-        off += kj < o.key ? cj : 0;
-      }
-      if (lane < m) p.run_off[r] = start + off;
+  constexpr int kSub = 8;
+  const int sub = threadIdx.x % kSub;
+  const int64_t ndest = (int64_t)p.nc * p.nc * p.nc, stride = (int64_t)gridDim.x * blockDim.x / kSub;
+  const int64_t d0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kSub;
+  for (int64_t it = 0; it < (ndest + stride - 1) / stride; it++) {  // the same for all lanes: the shuffles need the warp
+    const int64_t D = d0 + it * stride;
+    int s0 = 0, m = 0;
+    int64_t start = 0;
+    if (D < ndest) {
+      s0 = p.dest_start[D];
+      m = p.dest_start[D + 1] - s0;
+      if (m) start = p.cell_base_new[owner_ext_cell(p, (int32_t)D)];
+    }
+    const int r = sub < m ? p.run_list[s0 + sub] : 0;
+    DriftRun o;
+    o.key = ~0ull;
+    o.count = 0;
+    if (sub < m) o = p.runs[r];
+    int off = 0;
+#pragma unroll
+    for (int j = 0; j < kSub; j++) {
+      const uint64_t kj = __shfl_sync(0xffffffffu, o.key, j, kSub);
+      const int cj = __shfl_sync(0xffffffffu, o.count, j, kSub);
+      off += kj < o.key ? cj : 0;
+    }
+    if (m <= kSub) {
+      if (sub < m) p.run_off[r] = start + off;
       continue;
     }
-    for (int i = lane; i < m; i += 32) {
-      const int32_t r = p.run_list[s0 + i];
-      const uint64_t key = p.runs[r].key;
-      int64_t off = 0;
+    for (int i = sub; i < m; i += kSub) {
+      const int32_t ri = p.run_list[s0 + i];
+      const uint64_t key = p.runs[ri].key;
+      int64_t sum = 0;
       for (int j = 0; j < m; j++) {
-        const DriftRun o = p.runs[p.run_list[s0 + j]];
-        off += o.key < key ? o.count : 0;
+        const DriftRun q = p.runs[p.run_list[s0 + j]];
+        sum += q.key < key ? q.count : 0;
       }
-      p.run_off[r] = start + off;
+      p.run_off[ri] = start + sum;
     }
   }
 }
@@ -424,26 +432,35 @@ __global__ void __launch_bounds__(kDriftWarps * 32) k_drift_write(DriftK p) {
     if (n <= 0 || n >= (1 << kRankBits) - 1) continue;
     if (base < 0 || base + n > p.n_used) continue;
     const int rb = p.run_base[S];
-    for (int l = lane; l < n; l += 32) {
-      const int64_t ip = base + l;
-      const uint32_t w = p.runrank[ip];
-      // the copy's own data does not depend on its slot: loaded beside the slot lookup
+    for (int c0 = 0; c0 < n; c0 += 32) {
+      // the copy's slot (-1: dropped) ...
+      const int64_t ip = base + c0 + lane;
+      const uint32_t w = c0 + lane < n ? p.runrank[ip] : kDropped;
+      const int64_t id = p.pid && c0 + lane < n ? p.pid[ip] : 0;
+      // ... while the values of the 32 copies arrive one by one: value e = 3 copy + axis, three a lane, so that
+      // loads and (runs being contiguous) stores are coalesced
+      const int ne = 3 * min(32, n - c0);
+      const int64_t e0 = 3 * (base + c0);
       float v[3];
       int16_t x[3];
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        v[d] = p.vp[3 * ip + d];
-        x[d] = p.xp[3 * ip + d];
+      for (int k = 0; k < 3; k++) {
+        const int e = min(lane + 32 * k, ne - 1);
+        v[k] = p.vp[e0 + e];
+        x[k] = p.xp[e0 + e];
       }
-      const int64_t id = p.pid ? p.pid[ip] : 0;
-      if (w == kDropped) continue;
-      const int64_t pos = p.run_off[rb + (int)(w >> kRankBits)] + (int64_t)(w & ((1u << kRankBits) - 1u));
+      int pos = -1;
+      if (w != kDropped) pos = (int)(p.run_off[rb + (int)(w >> kRankBits)] + (int64_t)(w & ((1u << kRankBits) - 1u)));
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        p.xp_new[3 * pos + d] = drift_offset(p, x[d], v[d], p.err);
-        p.vp_new[3 * pos + d] = v[d];
+      for (int k = 0; k < 3; k++) {
+        const int e = lane + 32 * k, c = e / 3, d = e - 3 * c;
+        const int pc = __shfl_sync(0xffffffffu, pos, c);
+        if (e < ne && pc >= 0) {
+          p.xp_new[3 * (int64_t)pc + d] = drift_offset(p, x[k], v[k], p.err);
+          p.vp_new[3 * (int64_t)pc + d] = v[k];
+        }
       }
-      if (p.pid) p.pid_new[pos] = id;
+      if (p.pid && pos >= 0) p.pid_new[pos] = id;
     }
   }
 }
@@ -466,13 +483,39 @@ __global__ void __launch_bounds__(kDriftWarps * 32) k_halo_fill(DriftK p, const 
     mirrored_cell(p, t, cx, cy, cz, tt, l);
     const int64_t src = cell_base[ext_cell(p, tt, l)];
     if (dst < 0 || src < 0 || dst + n > p.n_used_new || src + n > p.n_used_new) continue;  // inconsistent spine
-    // the cell's arrays are contiguous on both sides: copied value by value, coalesced
-    for (int i = lane; i < 3 * n; i += 32) {
-      if (xp) xp[3 * dst + i] = xp[3 * src + i];
-      vp[3 * dst + i] = vp[3 * src + i];
+    // The cell's arrays are contiguous on both sides: copied value by value, coalesced, 64 copies a step with
+    // all its loads under way before the first store
+    for (int i0 = 0; i0 < 3 * n; i0 += 192) {
+      float v[6];
+      int16_t x[6];
+      int64_t id[2];
+#pragma unroll
+      for (int k = 0; k < 6; k++) {
+        const int i = i0 + lane + 32 * k;
+        if (i < 3 * n) {
+          v[k] = vp[3 * src + i];
+          if (xp) x[k] = xp[3 * src + i];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const int i = i0 / 3 + lane + 32 * k;
+        if (pid && i < n) id[k] = pid[src + i];
+      }
+#pragma unroll
+      for (int k = 0; k < 6; k++) {
+        const int i = i0 + lane + 32 * k;
+        if (i < 3 * n) {
+          vp[3 * dst + i] = v[k];
+          if (xp) xp[3 * dst + i] = x[k];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const int i = i0 / 3 + lane + 32 * k;
+        if (pid && i < n) pid[dst + i] = id[k];
+      }
     }
-    if (pid)
-      for (int i = lane; i < n; i += 32) pid[dst + i] = pid[src + i];
   }
 }
 
@@ -547,7 +590,7 @@ void launch_drift_place(const DriftArgs &a, int32_t nruns, int32_t *scan_tmp, cu
   const int64_t ndest = (int64_t)a.L->nc * a.L->nc * a.L->nc;
   scan_exclusive_i32(a.dest_runs, ndest, (int32_t *)a.dest_start, scan_tmp, s);
   if (nruns > 0) k_runs_fill<<<(unsigned)((nruns + 255) / 256), 256, 0, s>>>(p, nruns);
-  k_runs_order<<<warp_grid(ndest, a.num_sms), kDriftWarps * 32, 0, s>>>(p);
+  k_runs_order<<<warp_grid((ndest + 3) / 4, a.num_sms), kDriftWarps * 32, 0, s>>>(p);  // four cells a warp
   k_drift_write<<<warp_grid(p.ncells_src, a.num_sms), kDriftWarps * 32, 0, s>>>(p);
   k_halo_fill<<<warp_grid(p.ncells_src, a.num_sms), kDriftWarps * 32, 0, s>>>(p, a.rhoc_new, a.cell_base_new,
                                                                                  a.xp_new, a.vp_new, a.pid_new);
