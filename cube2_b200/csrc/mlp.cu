@@ -650,22 +650,27 @@ __device__ __forceinline__ bool wg_all(int wg, bool v) {
   return r != 0;
 }
 
-// 32 consecutive FP32 columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32]) {
-  uint32_t r[32];
+// 32 consecutive FP32 columns of this thread's TMEM lane, without waiting; tmem_wait32 makes the registers good (they pass through it, so that no use
+// moves ahead of the wait)
+__device__ __forceinline__ void tmem_ld32_start(uint32_t taddr, uint32_t r[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
         "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr)
       : "memory");
-#pragma unroll
-  for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
+}
+__device__ __forceinline__ void tmem_wait32(uint32_t r[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                 "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]),
+                 "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]),
+                 "+r"(r[30]), "+r"(r[31])::"memory");
 }
 
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float v[4]) {
@@ -822,19 +827,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_apply_tc(MlpApplyK p, int
       tc_fence_after();
       if (!ok) break;
       const float *b = bias + l * kMlpW;
+      // 32 columns at a time: enough independent GELUs to keep the special-function unit busy
 #pragma unroll 1
-      for (int c0 = 0; c0 < kMlpW; c0 += 16) {
-        float v[16];
-        tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
-        __align__(16) __nv_bfloat162 h[8];
+      for (int c0 = 0; c0 < kMlpW; c0 += 32) {
+        uint32_t r[32];
+        tmem_ld32_start(tmem + lane_base + (uint32_t)c0, r);
+        tmem_wait32(r);
+        __align__(16) __nv_bfloat162 h[16];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
+        for (int j = 0; j < 16; j++) {
           const float2 b2 = *reinterpret_cast<const float2 *>(b + c0 + 2 * j);
-          const float2 a = gelu2(__fadd2_rn(make_float2(v[2 * j], v[2 * j + 1]), b2));
+          const float2 a = gelu2(__fadd2_rn(make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), b2));
           h[j] = __floats2bfloat162_rn(a.x, a.y);
         }
 #pragma unroll
-        for (int c = 0; c < 2; c++)
+        for (int c = 0; c < 4; c++)
           *reinterpret_cast<uint4 *>(act + umma_off(m, c0 + 8 * c, kTcRows)) = reinterpret_cast<const uint4 *>(h)[c];
       }
     }
