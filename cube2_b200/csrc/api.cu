@@ -90,8 +90,12 @@ struct Ctx {
   cudaStream_t side2 = nullptr;
   cudaEvent_t ev_pm3done = nullptr, ev_join2 = nullptr;
   Buf xp, rhoc, idx, vp, cell_base;
-  Buf tiles, count, cell_start, scan_tmp, spos, spill, spill_rank, counters, items, range_loc, sched;
-  Buf rho, rhok, force, jobs, out;
+  Buf tiles;  // PP grids by tile, then PP ranges by subtile
+  Buf count, cell_start, scan_tmp, spos, spill, spill_rank, counters, items;
+  Buf rho, rhok, force, jobs;
+  // What a kick starts from zero, cleared by one memset: the outputs and status word (out), the binning's
+  // counters, the brick kernels' counters and the PP schedule, at the offsets below
+  Buf out;
   Buf mlp_pos, mlp_rho, mlp_n;  // learned shell: positions of the copies, fine-grid CIC density, listed copies
   // PP kernel shape: fixed (pp_fixed >= 0, cube_pp_set_shape) or autotuned, keyed by
   // pp_shape_key; pp_ms holds the last tuning's times, pp_last the shape of the last PP kick
@@ -111,7 +115,6 @@ struct Ctx {
   Buf ks_out;                  // FP64 conservation sums
   Buf fb_out;                  // learned-shell fallback statistics
   Buf phi_pad;                 // padded potential of the brick kernels
-  Buf brick_ctr;               // their work counter
   Buf dep_items;               // the brick deposit's work list
   cudaEvent_t tune_ev[2 * kMaxPPShapes] = {};
   void *h_stage = nullptr;  // pinned staging for small tables
@@ -439,6 +442,17 @@ static void fill_ptotal(const Meta &m, const int32_t *rhoc, double *ptotal) {
   }
 }
 
+// Words of g.out: [0..4] the outputs of a kick, [5] the device status word, [8..8 + 128) counters of the binning,
+// then the brick kernels' counters (a pair for each of kBrickCtrs launches), then the PP schedule.
+constexpr int kOutErr = 5, kOutCtr = 8, kOutBrick = kOutCtr + 128, kBrickCtrs = 64, kOutSched = kOutBrick + 2 * kBrickCtrs;
+static int32_t *out_word(int w) { return (int32_t *)g.out.p + w; }
+static int clear_outputs(cudaStream_t s) {
+  const size_t bytes = sizeof(int32_t) * (kOutSched + sched_ints(g.L.ntile));
+  CK(grow(g.out, bytes));
+  CU(cudaMemsetAsync(g.out.p, 0, bytes, s));
+  return CUBE_OK;
+}
+
 // ---------------------------------------------------------------------------------------------
 // pipeline stages (device pointers in ctx buffers or caller's)
 
@@ -522,9 +536,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     CK(grow(g.rho, sizeof(float) * n3 * nslots));
     CK(grow(g.rhok, sizeof(cufftComplex) * nk * nslots));
     const double scale = (double)L.rcs / (double)(1.0f / (float)rsf);
-    CK(grow(g.jobs, sizeof(MeshJob) * (size_t)L.ntile));
-    launch_mesh_jobs(L, scale, per_tile, (MeshJob *)g.jobs.p, g.stream);
-    g.launches += 1;
+    // (g.jobs, one job per tile, was written with the cell table)
     PM3Args a{};
     a.L = &g.L;
     a.rsf = rsf;
@@ -550,8 +562,11 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     a.vp = d.vp;
     a.out = (float *)g.out.p;
     a.want_vmax = want_vmax;
-    a.err = (int32_t *)g.counters.p + 2;
+    a.err = out_word(kOutErr);
     a.num_sms = g.num_sms;
+    a.brick_ctr = out_word(kOutBrick);
+    a.dep_count = out_word(kOutBrick + kBrickCtrs);
+    a.zeroed = true;
     // the force difference is fused into the gather brick by brick where the geometry allows;
     // otherwise the three force arrays are written and gathered from
     const bool fused = pm3_brick_mc(a) > 0;
@@ -563,8 +578,6 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
       CK(grow(g.phi_pad, sizeof(float) * m3 * nslots));
       a.phi = (float *)g.phi_pad.p;
       a.phi_pad = kPotPad;
-      CK(grow(g.brick_ctr, sizeof(int32_t) * 64));
-      a.brick_ctr = (int32_t *)g.brick_ctr.p;
     }
     {
       CK(grow(g.dep_items, pm3_dep_items_bytes((int64_t)a.rdep[0] * a.rdep[1] * a.rdep[2], a.njobs, d.n_used)));
@@ -592,6 +605,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
         CK(wait_xp(g.stream, k));
         at.jobs = (const MeshJob *)g.jobs.p + g.grp_lo[k];
         at.njobs = g.grp_lo[k + 1] - g.grp_lo[k];
+        at.dep_count = a.dep_count + k;
         g.launches += launch_pm3_deposit(at, g.stream);
       }
     } else {
@@ -626,6 +640,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
         CU(cudaStreamWaitEvent(g.stream, g.ev_vp[k], 0));
         at.jobs = (const MeshJob *)g.jobs.p + g.grp_lo[k];
         at.njobs = g.grp_lo[k + 1] - g.grp_lo[k];
+        at.brick_ctr = a.brick_ctr + k;
         gather(at);
         CU(cudaEventRecord(g.ev_ready[k], g.stream));
       }
@@ -687,7 +702,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
   // a stored copy is deposited into the meshes of at most 2 (subtiles of one cell: 3) subtiles per axis
   const int64_t ndep = d.n_used * (L.ntt > 1 ? 8 : 27);
   CK(grow(g.dep_items, pm3_dep_items_bytes((int64_t)(L.ntt + 2) * (L.ntt + 2) * (L.ntt + 2), L.ns3, ndep)));
-  CK(grow(g.brick_ctr, sizeof(int32_t) * 64));
+  int nbatch = 0;
   for (const Batch &bt : batches) {
     const int rsf = ratio_sf[bt.lev - 1], n = bt.n, nj = bt.nj;
     const int nfp = L.ntt * L.rcs * rsf, nfb = L.rcs * rsf;
@@ -729,9 +744,13 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     a.vp = d.vp;
     a.out = (float *)g.out.p;
     a.want_vmax = want_vmax;
-    a.err = (int32_t *)g.counters.p + 2;
+    a.err = out_word(kOutErr);
     a.num_sms = g.num_sms;
-    a.brick_ctr = (int32_t *)g.brick_ctr.p;
+    // each batch its own zeroed counters, while there are any; later batches clear the last ones
+    const int ctr = std::min(nbatch, kBrickCtrs - 1);
+    a.brick_ctr = out_word(kOutBrick + ctr);
+    a.dep_count = out_word(kOutBrick + kBrickCtrs + ctr);
+    a.zeroed = nbatch++ < kBrickCtrs;
     a.dep_items = (int2 *)g.dep_items.p;
     a.n_particles_hint = ndep;
     a.phi = a.rho;  // the potential in place, read by the brick gather where the geometry allows
@@ -788,7 +807,8 @@ static uint64_t pp_shape_key(const Meta &m, int64_t n_used) {
 // (work list + force kernel, kicking scratch velocities), twice, and the fastest by the better of
 // its two times is kept.  The binning has been enqueued on `st` already; the host waits for the
 // timings, once per key.  A kick being captured into a graph cannot wait and uses shape 0.
-static int choose_pp_shape(const Meta &m, int64_t n_used, PPArgs &p, cudaStream_t st) {
+// `tuned`: the schedule words hold a timing run's work list.
+static int choose_pp_shape(const Meta &m, int64_t n_used, PPArgs &p, cudaStream_t st, bool &tuned) {
   if (g.pp_fixed >= 0) {
     p.shape = g.pp_last = g.pp_fixed;
     return CUBE_OK;
@@ -839,6 +859,7 @@ static int choose_pp_shape(const Meta &m, int64_t n_used, PPArgs &p, cudaStream_
     if (best[k] < best[pick]) pick = k;
   }
   g.pp_tuned[key] = pick;
+  tuned = true;
   p.shape = g.pp_last = pick;
   return CUBE_OK;
 }
@@ -848,8 +869,13 @@ static int choose_pp_shape(const Meta &m, int64_t n_used, PPArgs &p, cudaStream_
 static int run_pp_prep(const Meta &m, const Dev &d, float mass, float kick, size_t &soff, PPArgs &p,
                        cudaStream_t st, unsigned long long *pairs) {
   const Lay &L = g.L;
-  CK(upload(g.tiles, m.tiles.data(), m.tiles.size(), soff, st));
-  CK(upload(g.range_loc, m.range_loc.data(), m.range_loc.size(), soff, st));
+  // the PP grids by tile and the PP ranges by subtile, in one table and one copy
+  const size_t tile_bytes = (sizeof(TilePP) * m.tiles.size() + 15) / 16 * 16;
+  std::vector<char> tab(tile_bytes + sizeof(float) * m.range_loc.size());
+  memcpy(tab.data(), m.tiles.data(), sizeof(TilePP) * m.tiles.size());
+  memcpy(tab.data() + tile_bytes, m.range_loc.data(), sizeof(float) * m.range_loc.size());
+  CK(upload(g.tiles, tab.data(), tab.size(), soff, st));
+  const float *d_range = (const float *)((const char *)g.tiles.p + tile_bytes);
   CK(grow(g.count, sizeof(int32_t) * (size_t)m.ncells));
   CK(grow(g.cell_start, sizeof(int32_t) * (size_t)(m.ncells + 1)));
   CK(grow(g.scan_tmp, sizeof(int32_t) * scan_tmp_elems(m.ncells)));
@@ -861,8 +887,7 @@ static int run_pp_prep(const Meta &m, const Dev &d, float mass, float kick, size
   for (auto &t : m.tiles) interior += (int64_t)L.nt * t.rcp * L.nt * t.rcp * L.nt * t.rcp;
   const int64_t item_cap = interior + d.n_used / pp_min_chunk() + 16;
   CK(grow(g.items, sizeof(PPItem) * (size_t)item_cap));
-  CK(grow(g.sched, sizeof(int32_t) * sched_ints(L.ntile)));
-  int32_t *ctr = (int32_t *)g.counters.p;  // [0] spill_n [2] err
+  int32_t *const err = out_word(kOutErr);
   BinArgs b{};
   b.L = &g.L;
   b.d_tiles = (const TilePP *)g.tiles.p;
@@ -876,13 +901,14 @@ static int run_pp_prep(const Meta &m, const Dev &d, float mass, float kick, size
   b.spos = (float4 *)g.spos.p;
   b.spill = (Spill *)g.spill.p;
   b.spill_rank = (int32_t *)g.spill_rank.p;
-  b.spill_n = ctr + 0;
+  b.spill_n = out_word(kOutCtr);
   b.spill_cap = spill_cap;
   b.scan_tmp = (int32_t *)g.scan_tmp.p;
-  b.err = ctr + 2;
+  b.err = err;
+  b.no_spill = pp_binning_spill_free(L, m.tiles.data());
   if (bin_smem_bytes(m.max_rcp) > 200 * 1024) return fail(CUBE_ERR_INVALID);  // rcp^3 histograms per warp
   b.spatial = 1;
-  if (g.xp_pending && pp_binning_spill_free(L, m.tiles.data())) {
+  if (g.xp_pending && b.no_spill) {
     // xp is arriving group by group: each group of tiles is binned as soon as its xp is in
     if (g.timing) CU(cudaEventRecord(g.ring[g.ring_cur][2], st));
     for (int k = 0; k < g.ngrp; k++) {
@@ -894,7 +920,7 @@ static int run_pp_prep(const Meta &m, const Dev &d, float mass, float kick, size
     CK(wait_xp(st));
     if (g.timing) CU(cudaEventRecord(g.ring[g.ring_cur][2], st));
     launch_pp_binning(b, st);
-    g.launches += 7;  // count, spill sort, 3 scan passes, scatter, spill placement
+    g.launches += b.no_spill ? 5 : 7;  // count, spill sort, 3 scan passes, scatter, spill placement
   }
   CU(cudaGetLastError());
   p = PPArgs{};
@@ -904,21 +930,22 @@ static int run_pp_prep(const Meta &m, const Dev &d, float mass, float kick, size
   p.ncells = m.ncells;
   p.cell_start = (const int32_t *)g.cell_start.p;
   p.spos = (const float4 *)g.spos.p;
-  p.range_loc = (const float *)g.range_loc.p;
+  p.range_loc = d_range;
   p.items = (PPItem *)g.items.p;
-  p.sched = (int32_t *)g.sched.p;
+  p.sched = out_word(kOutSched);
   p.item_cap = item_cap;
   p.vp = d.vp;
   p.mass2 = mass * mass;
   p.kick = kick;
   p.out = (float *)g.out.p;
   p.want_vmax = 1;
-  p.err = ctr + 2;
+  p.err = err;
   p.num_sms = g.num_sms;
   p.pairs = pairs;
   p.shape = 0;
-  if (!pairs) CK(choose_pp_shape(m, d.n_used, p, st));
-  launch_pp_items(p, st);
+  bool tuned = false;
+  if (!pairs) CK(choose_pp_shape(m, d.n_used, p, st, tuned));
+  launch_pp_items(p, st, !tuned);
   g.launches += 3;
   CU(cudaGetLastError());
   if (g.timing) CU(cudaEventRecord(g.ring[g.ring_cur][6], st));
@@ -999,13 +1026,10 @@ static int run_kick(const int32_t *ires, const int32_t *ixyz3, const int32_t *ra
   // the subtile geometry uploads one mesh job per subtile
   CK(stage_begin(((size_t)4 << 20) + (g.L.pm3_mode == CUBE_PM3_SUBTILE ? sizeof(MeshJob) * (size_t)g.L.ns3 : 0)));
   CK(grow(g.cell_base, sizeof(int64_t) * (size_t)g.L.ntile * g.L.nte * g.L.nte * g.L.nte));
-  CK(grow(g.out, sizeof(float) * 8));
-  CK(grow(g.counters, sizeof(int32_t) * 128));
   size_t soff = 0;
   // kick coefficient a_mid*dt/6/pi (kick.f90:529, pp_force_kernel.c:355)
   const float kick = (float)((double)(a_mid * dt / 6.0f) / 3.14159265358979323846);
-  CU(cudaMemsetAsync(g.out.p, 0, sizeof(float) * 8, g.stream));
-  CU(cudaMemsetAsync(g.counters.p, 0, sizeof(int32_t) * 128, g.stream));
+  CK(clear_outputs(g.stream));
   if (g.timing) {
     g.ring_cur = g.ring_next;
     g.ring_next = (g.ring_next + 1) % Ctx::kRing;
@@ -1014,7 +1038,11 @@ static int run_kick(const int32_t *ires, const int32_t *ixyz3, const int32_t *ra
     g.ring_pp[g.ring_cur] = do_pp;
     CU(cudaEventRecord(g.ring[g.ring_cur][0], g.stream));
   }
-  launch_cell_table(g.L, d.rhoc, d.idx, (int64_t *)g.cell_base.p, g.stream);
+  const bool periodic = do_pm3 && g.L.pm3_mode != CUBE_PM3_SUBTILE;
+  if (periodic) CK(grow(g.jobs, sizeof(MeshJob) * (size_t)g.L.ntile));
+  const int rsf0 = ratio_sf[m.ires_loc[0] - 1];  // the periodic geometries have one level (run_pm3 checks)
+  launch_cell_table_jobs(g.L, d.rhoc, d.idx, (int64_t *)g.cell_base.p, (double)g.L.rcs / (double)(1.0f / (float)rsf0),
+                         g.L.pm3_mode == CUBE_PM3_TILE_PERIODIC, periodic ? (MeshJob *)g.jobs.p : nullptr, g.stream);
   g.launches += 1;
   CU(cudaGetLastError());
   if (do_pm3 && do_pp) {
@@ -1040,9 +1068,6 @@ static int run_kick(const int32_t *ires, const int32_t *ixyz3, const int32_t *ra
   }
   if (g.timing) CU(cudaEventRecord(g.ring[g.ring_cur][5], g.stream));
   CK(stage_end());
-  // error word next to the outputs
-  CU(cudaMemcpyAsync((char *)g.out.p + 5 * sizeof(float), (char *)g.counters.p + 2 * sizeof(int32_t),
-                     sizeof(int32_t), cudaMemcpyDeviceToDevice, g.stream));
   return CUBE_OK;
 }
 
@@ -1268,11 +1293,11 @@ int cube_pp_work_stats(int64_t out[4]) {
   if (!out) return fail(CUBE_ERR_INVALID);
   for (int k = 0; k < 4; k++) out[k] = 0;
   if (!g.configured) return fail(CUBE_ERR_NOT_CONFIGURED);
-  if (!g.items.p || !g.sched.p) return CUBE_OK;  // no PP kick yet
+  const size_t total_at = kOutSched + (size_t)sched_total_index(g.L.ntile);
+  if (!g.items.p || g.out.cap < sizeof(int32_t) * (total_at + 1)) return CUBE_OK;  // no PP kick yet
   CU(cudaDeviceSynchronize());
   int32_t n = 0;
-  CU(cudaMemcpy(&n, (const int32_t *)g.sched.p + sched_total_index(g.L.ntile), sizeof(int32_t),
-                cudaMemcpyDeviceToHost));
+  CU(cudaMemcpy(&n, out_word((int)total_at), sizeof(int32_t), cudaMemcpyDeviceToHost));
   const size_t cap = g.items.cap / sizeof(PPItem);
   if (n < 0 || (size_t)n > cap) return fail(CUBE_ERR_CAPACITY);
   std::vector<PPItem> it((size_t)n);
@@ -1947,8 +1972,7 @@ static int mlp_density(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const in
   CK(grow(g.mlp_rho, sizeof(float) * (size_t)ng3));
   CK(grow(g.mlp_n, sizeof(unsigned long long)));
   CK(grow(g.jobs, sizeof(MeshJob) * (size_t)L.ntile));
-  launch_mesh_jobs(L, (double)L.rcs, false, (MeshJob *)g.jobs.p, s);
-  launch_cell_table(L, d_rhoc, d_idx_b_r, (int64_t *)g.cell_base.p, s);
+  launch_cell_table_jobs(L, d_rhoc, d_idx_b_r, (int64_t *)g.cell_base.p, (double)L.rcs, false, (MeshJob *)g.jobs.p, s);
   CU(cudaMemsetAsync(g.mlp_rho.p, 0, sizeof(float) * ng3, s));
   PM3Args a{};  // the fine grid as a mesh of ratio_cs points per coarse cell
   a.L = &g.L;
@@ -1980,7 +2004,7 @@ static int mlp_density(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const in
     g.launches += 1;
   }
   launch_mlp_log1p((float *)g.mlp_rho.p, ng3, s);
-  g.launches += 3;
+  g.launches += 2;
   CU(cudaGetLastError());
   return CUBE_OK;
 }
@@ -2197,7 +2221,6 @@ void c_pm3_fft_finalize(void) {
   release(g.rhok);
   release(g.force);
   release(g.phi_pad);
-  release(g.brick_ctr);
   release(g.dep_items);
   release(g.jobs);
   release(g.mlp_pos);
@@ -2211,7 +2234,7 @@ void c_gpu_velocity_finalize(void) {
   cudaSetDevice(g.device);
   cudaStreamSynchronize(g.stream);
   Buf *bufs[] = {&g.xp, &g.rhoc, &g.idx, &g.vp, &g.cell_base, &g.tiles, &g.count, &g.cell_start, &g.scan_tmp,
-                 &g.spos, &g.spill, &g.spill_rank, &g.counters, &g.items, &g.range_loc, &g.sched, &g.out, &g.ks_out, &g.fb_out};
+                 &g.spos, &g.spill, &g.spill_rank, &g.counters, &g.items, &g.out, &g.ks_out, &g.fb_out};
   for (Buf *b : bufs) release(*b);
 }
 
@@ -2347,23 +2370,20 @@ int cube_pp_pair_count(const int32_t *ires, const int32_t *ixyz3, const float *a
   CK(grow(g.rhoc, sizeof(int32_t) * (size_t)nrows * L.nte));
   CK(grow(g.idx, sizeof(int64_t) * (size_t)nrows));
   CK(grow(g.cell_base, sizeof(int64_t) * (size_t)nrows * L.nte));
-  CK(grow(g.counters, sizeof(int32_t) * 128));
-  CK(grow(g.out, sizeof(float) * 8));
   CU(cudaMemcpyAsync(g.rhoc.p, rhoc, sizeof(int32_t) * nrows * L.nte, cudaMemcpyHostToDevice, g.stream));
   CU(cudaMemcpyAsync(g.idx.p, idx_b_r, sizeof(int64_t) * nrows, cudaMemcpyHostToDevice, g.stream));
   if (n_used) CU(cudaMemcpyAsync(g.xp.p, xp, sizeof(int16_t) * 3 * n_used, cudaMemcpyHostToDevice, g.stream));
-  CU(cudaMemsetAsync(g.counters.p, 0, sizeof(int32_t) * 128, g.stream));
-  CU(cudaMemsetAsync(g.out.p, 0, sizeof(float) * 8, g.stream));
+  CK(clear_outputs(g.stream));
   launch_cell_table(L, (const int32_t *)g.rhoc.p, (const int64_t *)g.idx.p, (int64_t *)g.cell_base.p, g.stream);
   Dev d{(const int16_t *)g.xp.p, (const int32_t *)g.rhoc.p, (const int64_t *)g.idx.p, nullptr, n_used};
   size_t soff = 0;
-  unsigned long long *d_pairs = (unsigned long long *)((int32_t *)g.counters.p + 8);
+  unsigned long long *d_pairs = (unsigned long long *)out_word(kOutCtr + 8);
   CK(run_pp(m, d, 1.0f, 0.0f, soff, d_pairs));
   CK(stage_end());
   unsigned long long h = 0;
   int32_t err = 0;
   CU(cudaMemcpyAsync(&h, d_pairs, sizeof(h), cudaMemcpyDeviceToHost, g.stream));
-  CU(cudaMemcpyAsync(&err, (int32_t *)g.counters.p + 2, sizeof(err), cudaMemcpyDeviceToHost, g.stream));
+  CU(cudaMemcpyAsync(&err, out_word(kOutErr), sizeof(err), cudaMemcpyDeviceToHost, g.stream));
   CU(cudaStreamSynchronize(g.stream));
   CK(check_err_word(err));
   *pairs = (int64_t)h;

@@ -29,9 +29,27 @@
 
 namespace cube {
 
+struct JobsK {
+  MeshJob *jobs;  // null: none
+  int ntile, nnt, nt, ncb, per_tile;
+  double scale;
+};
+
 __global__ void k_cell_table(int64_t nrows, int nte, const int32_t *__restrict__ rhoc,
-                             const int64_t *__restrict__ idx_b_r, int64_t *__restrict__ cell_base) {
+                             const int64_t *__restrict__ idx_b_r, int64_t *__restrict__ cell_base, JobsK jk) {
   int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (jk.jobs && r < jk.ntile) {  // a tile has more rows than one
+    const int t = (int)r, tc[3] = {t % jk.nnt, (t / jk.nnt) % jk.nnt, t / (jk.nnt * jk.nnt)};
+    MeshJob J;
+    J.t = t;
+    J.slot = jk.per_tile ? t : 0;
+    J.range = 0.f;
+    for (int q = 0; q < 3; q++) {
+      J.lo[q] = J.alo[q] = jk.ncb;
+      J.off[q] = jk.per_tile ? 0.0 : -(double)tc[q] * jk.nt * jk.scale;
+    }
+    jk.jobs[t] = J;
+  }
   if (r >= nrows) return;
   const int32_t *row = rhoc + r * nte;
   int64_t s = idx_b_r[r];
@@ -43,8 +61,14 @@ __global__ void k_cell_table(int64_t nrows, int nte, const int32_t *__restrict__
 
 void launch_cell_table(const Lay &L, const int32_t *rhoc, const int64_t *idx_b_r, int64_t *cell_base,
                        cudaStream_t s) {
-  int64_t nrows = (int64_t)L.ntile * L.nte * L.nte;
-  k_cell_table<<<(unsigned)((nrows + 255) / 256), 256, 0, s>>>(nrows, L.nte, rhoc, idx_b_r, cell_base);
+  launch_cell_table_jobs(L, rhoc, idx_b_r, cell_base, 0.0, false, nullptr, s);
+}
+
+void launch_cell_table_jobs(const Lay &L, const int32_t *rhoc, const int64_t *idx_b_r, int64_t *cell_base, double scale,
+                            bool per_tile, MeshJob *jobs, cudaStream_t s) {
+  const int64_t nrows = (int64_t)L.ntile * L.nte * L.nte;
+  const JobsK jk{jobs, L.ntile, L.nnt, L.nt, L.ncb, per_tile ? 1 : 0, scale};
+  k_cell_table<<<(unsigned)((nrows + 255) / 256), 256, 0, s>>>(nrows, L.nte, rhoc, idx_b_r, cell_base, jk);
 }
 
 struct BinK {
@@ -546,12 +570,12 @@ void launch_pp_binning(const BinArgs &a, cudaStream_t s) {
   const int64_t warps = (int64_t)p.ntile * p.R3;
   const unsigned blocks = (unsigned)((warps + kWarps - 1) / kWarps);
   const size_t shm = sizeof(int32_t) * kWarps * p.hist_words;
-  cudaMemsetAsync(a.spill_n, 0, sizeof(int32_t), s);
+  if (!a.no_spill) cudaMemsetAsync(a.spill_n, 0, sizeof(int32_t), s);
   k_pp_bin<false><<<blocks, kWarps * 32, shm, s>>>(p);
-  k_spill_fix<<<1, 1024, 0, s>>>(a.spill, a.spill_rank, a.spill_n, p.spill_cap, a.count);
+  if (!a.no_spill) k_spill_fix<<<1, 1024, 0, s>>>(a.spill, a.spill_rank, a.spill_n, p.spill_cap, a.count);
   scan_exclusive_i32(a.count, a.ncells, a.cell_start, a.scan_tmp, s);
   k_pp_bin<true><<<blocks, kWarps * 32, shm, s>>>(p);
-  k_spill_place<<<8, 256, 0, s>>>(p);
+  if (!a.no_spill) k_spill_place<<<8, 256, 0, s>>>(p);
 }
 
 bool pp_binning_spill_free(const Lay &L, const TilePP *h_tiles) {

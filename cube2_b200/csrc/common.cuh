@@ -140,6 +140,10 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 // cell_base[t][k][j][i] = idx_b_r[t][k][j] - sum(rhoc[t][k][j][i:])  (pp_force_kernel.c:203-209)
 void launch_cell_table(const Lay &L, const int32_t *rhoc, const int64_t *idx_b_r, int64_t *cell_base,
                        cudaStream_t s);
+// the same, and the mesh jobs of the periodic geometries: one mesh over the image, or one per tile (written
+// on the device, so that no host table has to cross)
+void launch_cell_table_jobs(const Lay &L, const int32_t *rhoc, const int64_t *idx_b_r, int64_t *cell_base, double scale,
+                            bool per_tile, MeshJob *jobs, cudaStream_t s);
 
 // PP binning (counting sort by PP cell, bit-exact with pp_force_kernel.c:196-274)
 struct BinArgs {
@@ -160,6 +164,7 @@ struct BinArgs {
   int32_t *scan_tmp;      // scan scratch
   int32_t *err;           // device error word
   int spatial;            // 1: order inside each PP cell by Morton sub-cell (kick); 0: reference order
+  bool no_spill = false;  // pp_binning_spill_free and *spill_n already 0: the spill passes are left out
 };
 void launch_pp_binning(const BinArgs &a, cudaStream_t s);
 // No particle can spill into the next coarse cell's PP cells (exact float keys); then the
@@ -220,8 +225,8 @@ int64_t sched_total_index(int ntile);  // where the work list's item count lies 
 int pp_num_shapes();
 PPShapeDesc pp_shape_desc(int i);
 int pp_min_chunk();  // smallest chunk of any shape: the work list capacity is sized for it
-// work list for the shape a.shape (shape 0 with a.pairs)
-void launch_pp_items(const PPArgs &a, cudaStream_t s);
+// work list for the shape a.shape (shape 0 with a.pairs); `zeroed`: a.sched is already zero
+void launch_pp_items(const PPArgs &a, cudaStream_t s, bool zeroed = false);
 // force kernel over the items of tiles [t_lo, t_hi) (t_hi < 0: all tiles); disjoint tile ranges
 // and the full range have their own queue heads, so launches over disjoint ranges may run on
 // several streams
@@ -255,15 +260,15 @@ struct PM3Args {
   int num_sms = 148;
   float *phi = nullptr;      // potential of the brick gather, [nslots][(n + 2 phi_pad)^3]
   int phi_pad = 0;           // its ghost points per side: kPotPad (periodic images), or 0 on buffered meshes
-  int32_t *brick_ctr = nullptr;  // work counter of the brick kernels (one int, zeroed by the launcher)
+  int32_t *brick_ctr = nullptr;  // work counter of the brick gather (one int)
+  int32_t *dep_count = nullptr;  // length of the deposit work list (one int; null: kept behind dep_items)
+  bool zeroed = false;           // both are already 0; otherwise the launchers clear them
   int2 *dep_items = nullptr;      // deposit work list: pm3_dep_items_bytes(...) of scratch
   int64_t n_particles_hint = 0;   // stored particles (sizes the deposit work list)
 };
 // scratch of the deposit work list for a launch over `njobs` jobs of `cells` coarse cells each
 size_t pm3_dep_items_bytes(int64_t cells_per_job, int njobs, int64_t n_used);
 constexpr int kPotPad = 4;  // ghost points per side of the padded potential of the brick kernels
-// mesh jobs of the periodic geometries: one mesh over the image, or one per tile
-void launch_mesh_jobs(const Lay &L, double scale, bool per_tile, MeshJob *jobs, cudaStream_t s);
 int launch_pm3_deposit(const PM3Args &a, cudaStream_t s);  // returns the kernels it launched
 // CIC instead of TSC on the brick kernels' geometry (pm3_brick_mc != 0, else nothing and 0): cell-centred points
 int launch_cic_bricks(const PM3Args &a, cudaStream_t s);

@@ -1253,26 +1253,6 @@ size_t pm3_dep_items_bytes(int64_t cells_per_job, int njobs, int64_t n_used) {
   return sizeof(int2) * ((size_t)cells_per_job * njobs + (size_t)(n_used / kDepChunk) + 2);
 }
 
-// Mesh jobs of the periodic geometries, one per tile: written on the device, so that no host table has to cross
-// (and a captured call replays from nothing but device memory)
-__global__ void k_mesh_jobs(MeshJob *jobs, int ntile, int nnt, int nt, int ncb, double scale, int per_tile) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntile; t += gridDim.x * blockDim.x) {
-    const int tc[3] = {t % nnt, (t / nnt) % nnt, t / (nnt * nnt)};
-    MeshJob J;
-    J.t = t;
-    J.slot = per_tile ? t : 0;
-    J.range = 0.f;
-    for (int q = 0; q < 3; q++) {
-      J.lo[q] = J.alo[q] = ncb;
-      J.off[q] = per_tile ? 0.0 : -(double)tc[q] * nt * scale;
-    }
-    jobs[t] = J;
-  }
-}
-void launch_mesh_jobs(const Lay &L, double scale, bool per_tile, MeshJob *jobs, cudaStream_t s) {
-  k_mesh_jobs<<<(unsigned)std::min((L.ntile + 127) / 128, 148), 128, 0, s>>>(jobs, L.ntile, L.nnt, L.nt, L.ncb, scale, per_tile);
-}
-
 // the brick deposit (TSC or CIC), with its work list where the caller gives the scratch for one
 template <bool CIC>
 static int launch_deposit_bricks(const PM3Args &a, int mc, cudaStream_t s) {
@@ -1287,8 +1267,8 @@ static int launch_deposit_bricks(const PM3Args &a, int mc, cudaStream_t s) {
   }
   // at most one item per brick plus one per kDepChunk particles
   const int64_t cap = nbricks + a.n_particles_hint / kDepChunk + 1;
-  int *count = reinterpret_cast<int *>(a.dep_items + cap);
-  cudaMemsetAsync(count, 0, sizeof(int), s);
+  int *count = a.dep_count ? a.dep_count : reinterpret_cast<int *>(a.dep_items + cap);
+  if (!a.dep_count || !a.zeroed) cudaMemsetAsync(count, 0, sizeof(int), s);
   k_dep_items<<<(unsigned)std::min<int64_t>((nbricks + 255) / 256, 4096), 256, 0, s>>>(p, mc, nbricks, kDepChunk,
                                                                                      a.dep_items, count, cap);
   k_deposit_brick<CIC><<<(unsigned)std::min(cap, resident), kDepThreads, 0, s>>>(p, mc, a.dep_items, count, (int)cap);
@@ -1345,7 +1325,7 @@ bool launch_pm3_force_gather(const PM3Args &a, cudaStream_t s) {
   set_smem_attr_once((const void *)k_force_gather, kFgSmem);
   const int64_t grid = std::min<int64_t>(nbricks, a.num_sms > 0 ? a.num_sms : 148);
   if (!a.brick_ctr) return false;
-  cudaMemsetAsync(a.brick_ctr, 0, sizeof(int32_t), s);
+  if (!a.zeroed) cudaMemsetAsync(a.brick_ctr, 0, sizeof(int32_t), s);
   if (grid > 0) k_force_gather<<<(unsigned)grid, kFgThreads, kFgSmem, s>>>(p, mc, nbricks, a.phi_pad, tmap);
   return true;
 }

@@ -1111,9 +1111,9 @@ static void launch_items_c(const PPK &p, dim3 grid, cudaStream_t s, int32_t *sch
   k_pp_items<1, C><<<grid, 256, 0, s>>>(p);
 }
 
-void launch_pp_items(const PPArgs &a, cudaStream_t s) {
+void launch_pp_items(const PPArgs &a, cudaStream_t s, bool zeroed) {
   PPK p = make_ppk(a);
-  cudaMemsetAsync(a.sched, 0, sizeof(int32_t) * sched_ints(a.L->ntile), s);
+  if (!zeroed) cudaMemsetAsync(a.sched, 0, sizeof(int32_t) * sched_ints(a.L->ntile), s);
   dim3 grid((unsigned)((p.max_cells + 255) / 256), (unsigned)a.L->ntile);
   switch (pp_shape_desc(a.pairs ? 0 : a.shape).chunk) {
     case 16: launch_items_c<16>(p, grid, s, a.sched, a.L->ntile); break;
