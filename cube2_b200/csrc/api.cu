@@ -96,7 +96,8 @@ struct Ctx {
   // What a kick starts from zero, cleared by one memset: the outputs and status word (out), the binning's
   // counters, the brick kernels' counters and the PP schedule, at the offsets below
   Buf out;
-  Buf mlp_pos, mlp_rho, mlp_n;  // learned shell: positions of the copies, fine-grid CIC density, listed copies
+  // learned shell: positions of the copies, fine-grid CIC density, listed copies, stencil rows of the density
+  Buf mlp_pos, mlp_rho, mlp_n, mlp_tab;
   // PP kernel shape: fixed (pp_fixed >= 0, cube_pp_set_shape) or autotuned, keyed by
   // pp_shape_key; pp_ms holds the last tuning's times, pp_last the shape of the last PP kick
   int pp_fixed = -1;
@@ -1960,7 +1961,7 @@ int cube_mlp_get_params(cube_mlp *h, float *params, float *grads) {
   return CUBE_OK;
 }
 
-// log(1 + density) on the fine grid of the image, on g.stream.  With `list`, the interior copies are listed in
+// The CIC density on the fine grid of the image, on g.stream.  With `list`, the interior copies are listed in
 // g.mlp_pos (g.mlp_n of them).
 static int mlp_density(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const int16_t *d_xp, int64_t n_used, bool list) {
   const Lay &L = g.L;
@@ -2003,8 +2004,7 @@ static int mlp_density(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const in
     launch_mlp_cic((const float4 *)g.mlp_pos.p, (const unsigned long long *)g.mlp_n.p, L.ng, (float *)g.mlp_rho.p, s);
     g.launches += 1;
   }
-  launch_mlp_log1p((float *)g.mlp_rho.p, ng3, s);
-  g.launches += 2;
+  g.launches += 1;
   CU(cudaGetLastError());
   return CUBE_OK;
 }
@@ -2028,8 +2028,9 @@ int cube_mlp_features(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const int
   const StreamScope scope(stream);
   cudaStream_t s = g.stream;
   CK(mlp_density(d_rhoc, d_idx_b_r, d_xp, n_used, false));
+  launch_mlp_log1p((float *)g.mlp_rho.p, (int64_t)g.L.ng * g.L.ng * g.L.ng, s);
   launch_mlp_pos(g.L, d_xp, d_rhoc, (const int64_t *)g.cell_base.p, (float4 *)g.mlp_pos.p, s);
-  g.launches += 1;
+  g.launches += 2;
   launch_mlp_features((const float4 *)g.mlp_pos.p, n_used, (const float *)g.mlp_rho.p, g.L.ng,
                       (__nv_bfloat16 *)d_X, s);
   g.launches += 1;
@@ -2066,12 +2067,13 @@ int cube_mlp_kick(cube_mlp *h, const int32_t *d_rhoc, const int64_t *d_idx_b_r, 
   CK(ensure_device());
   const StreamScope scope(stream);
   cudaStream_t s = g.stream;
+  CK(grow(g.mlp_tab, sizeof(uint2) * (size_t)g.L.ng * g.L.ng * g.L.ng));
   CK(mlp_density(d_rhoc, d_idx_b_r, d_xp, n_used, true));
   // the kick coefficient of run_kick (kick.f90:529), times the network's output scale
   const float kick = (float)((double)(a_mid * dt / 6.0f) / 3.14159265358979323846);
-  launch_mlp_apply(h->p, (const float4 *)g.mlp_pos.p, (const unsigned long long *)g.mlp_n.p,
-                   (const float *)g.mlp_rho.p, g.L.ng, d_vp, kick * scale, g.num_sms, s);
-  g.launches += 1;
+  launch_mlp_apply(h->p, (const float4 *)g.mlp_pos.p, (const unsigned long long *)g.mlp_n.p, (float *)g.mlp_rho.p,
+                   g.mlp_tab.p, g.L.ng, d_vp, kick * scale, g.num_sms, s);
+  g.launches += 2;
   CU(cudaGetLastError());
   // the inference kernel's bounded waits report through a status word: read it once the kick is done
   int32_t e = 0;
@@ -2226,6 +2228,7 @@ void c_pm3_fft_finalize(void) {
   release(g.mlp_pos);
   release(g.mlp_rho);
   release(g.mlp_n);
+  release(g.mlp_tab);
 }
 
 void c_gpu_velocity_finalize(void) {

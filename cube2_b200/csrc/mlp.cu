@@ -421,12 +421,30 @@ constexpr size_t kApplySmem = sizeof(bf16) * ((size_t)kMlpW * kLd1 + 2 * (size_t
                               sizeof(float) * (3 * kMlpW + 8) +
                               sizeof(bf16) * (size_t)kApplyWarps * 16 * (kLd1 + 2 * kLdW);
 
+// The stencil rows of the network's input as one load each: tab[(z ng + y) ng + x] holds log(1 + rho) of cells
+// x .. x + 3 (periodic) of row (y, z), rounded to BF16 as the input is.  A block takes 256 cells of a row.  It also takes the logarithm's own pass
+// over the density.  Bound by its writes (8 bytes a cell: 57 MB at 192^3, 40 us, cold); the inference
+// kernel went from 1410 to 1203 us with it.
+constexpr int kTabCells = 256;
+__global__ void __launch_bounds__(kTabCells) k_mlp_table(const float *rho, int ng, uint2 *tab) {
+  __shared__ uint16_t s[kTabCells + 3];
+  const int64_t row = (int64_t)blockIdx.y * gridDim.z + blockIdx.z;
+  const int x0 = blockIdx.x * kTabCells, len = min(kTabCells, ng - x0);
+  const float *r = rho + row * ng;
+  for (int i = threadIdx.x; i < len + 3; i += kTabCells)
+    s[i] = __bfloat16_as_ushort(__float2bfloat16_rn(log1pf(r[(x0 + i) % ng])));
+  __syncthreads();
+  const int i = threadIdx.x;
+  if (i < len) tab[row * ng + x0 + i] = make_uint2(s[i] | (uint32_t)s[i + 1] << 16, s[i + 2] | (uint32_t)s[i + 3] << 16);
+}
+
 struct MlpApplyK {
   const bf16 *wb;
   const float *master;
   const float4 *list;  // interior copies: fine position, w = storage index
   const unsigned long long *n_list;
-  const float *rho;
+  const float *rho;   // log(1 + density) per fine cell (k_mlp_apply)
+  const uint2 *tab;   // k_mlp_table's stencil rows (k_mlp_apply_tc)
   int ng;
   float *vp;
   float coef;  // kick coefficient times the output scale
@@ -701,8 +719,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
 
 // the inputs of mlp_inputs written straight into row m of the activation buffer, one 8-value
 // chunk at a time: chunk 2 dz + h holds the stencil rows dy = 2h - 1, 2h of plane dz (x fastest),
-// chunk 8 the offsets, chunk 9 zeros
-__device__ __forceinline__ void tc_inputs(float4 q, bool live, const float *__restrict__ rho, int ng,
+// chunk 8 the offsets, chunk 9 zeros.  A row is one 8-byte load of the table (64 scattered 4-byte loads and
+// as many conversions a particle before: the kernel's L1 was 65 % busy with them)
+__device__ __forceinline__ void tc_inputs(float4 q, bool live, const uint2 *__restrict__ tab, int ng,
                                           unsigned char *act, int m) {
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   if (!live) {
@@ -719,23 +738,21 @@ __device__ __forceinline__ void tc_inputs(float4 q, bool live, const float *__re
     i0[d] = (int)fl;
     f[d] = xs[d] - fl;
   }
-  int X[4];
+  const uint2 *const col = tab + wrap_cell(wrap_cell(i0[0] - 1, ng), ng);
+  int Y[4];
 #pragma unroll
-  for (int dx = 0; dx < 4; dx++) X[dx] = wrap_cell(i0[0] + dx - 1, ng);
-#pragma unroll 4
-  for (int c = 0; c < 8; c++) {  // 32 loads in flight
-    const int dz = c >> 1, h = c & 1;
+  for (int dy = 0; dy < 4; dy++) Y[dy] = wrap_cell(wrap_cell(i0[1] + dy - 1, ng), ng);
+  uint2 v[16];
+#pragma unroll
+  for (int dz = 0; dz < 4; dz++) {
     const int64_t Z = wrap_cell(wrap_cell(i0[2] + dz - 1, ng), ng);
-    __align__(16) __nv_bfloat162 v[4];
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int64_t Y = wrap_cell(wrap_cell(i0[1] + 2 * h + r - 1, ng), ng);
-      const float *row = rho + (Z * ng + Y) * ng;
-      v[2 * r] = __floats2bfloat162_rn(__ldg(row + X[0]), __ldg(row + X[1]));
-      v[2 * r + 1] = __floats2bfloat162_rn(__ldg(row + X[2]), __ldg(row + X[3]));
-    }
-    *reinterpret_cast<uint4 *>(act + umma_off(m, 8 * c, kTcRows)) = *reinterpret_cast<const uint4 *>(v);
+    for (int dy = 0; dy < 4; dy++) v[4 * dz + dy] = __ldg(col + (Z * ng + Y[dy]) * ng);
   }
+#pragma unroll
+  for (int c = 0; c < 8; c++)
+    *reinterpret_cast<uint4 *>(act + umma_off(m, 8 * c, kTcRows)) =
+        make_uint4(v[2 * c].x, v[2 * c].y, v[2 * c + 1].x, v[2 * c + 1].y);
   __align__(16) __nv_bfloat162 o[4];
   o[0] = __floats2bfloat162_rn(f[0], f[1]);
   o[1] = __floats2bfloat162_rn(f[2], 0.f);
@@ -811,7 +828,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_apply_tc(MlpApplyK p, int
     const int64_t i = tile * kTcRows + m;
     const bool live = i < n;
     const float4 q = live ? p.list[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    tc_inputs(q, live, p.rho, p.ng, act, m);  // layer-1 input row of this particle
+    tc_inputs(q, live, p.tab, p.ng, act, m);  // layer-1 input row of this particle
     // layers 1-3 (N = 128): MMA, then bias + GELU + BF16 back into the activation buffer
 #pragma unroll 1
     for (int l = 0; l < 3 && ok; l++) {
@@ -1371,18 +1388,21 @@ void launch_gemm_nt(const bf16 *A, int lda, const bf16 *B, int ldb, int M, int N
   k_gemm_nt<<<grid, 128, 0, s>>>(A, lda, B, ldb, M, N, K, bias, Z, ldz, H, ldh, act);
 }
 
-void launch_mlp_apply(const MlpParams &m, const float4 *list, const unsigned long long *n_list, const float *rho, int ng,
-                      float *vp, float coef, int num_sms, cudaStream_t s) {
+void launch_mlp_apply(const MlpParams &m, const float4 *list, const unsigned long long *n_list, float *rho, void *tab,
+                      int ng, float *vp, float coef, int num_sms, cudaStream_t s) {
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(k_mlp_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kApplySmem);
     cudaFuncSetAttribute(k_mlp_apply_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
     attr = true;
   }
-  MlpApplyK p{m.wb, m.master, list, n_list, rho, ng, vp, coef};
+  MlpApplyK p{m.wb, m.master, list, n_list, rho, (const uint2 *)tab, ng, vp, coef};
   if (getenv("CUBE_MLP_MMA_SYNC")) {
+    launch_mlp_log1p(rho, (int64_t)ng * ng * ng, s);
     k_mlp_apply<<<num_sms, kApplyWarps * 32, kApplySmem, s>>>(p);
   } else {
+    const dim3 grid((unsigned)((ng + kTabCells - 1) / kTabCells), (unsigned)ng, (unsigned)ng);
+    k_mlp_table<<<grid, kTabCells, 0, s>>>(rho, ng, (uint2 *)tab);
     k_mlp_apply_tc<<<num_sms, kTcThreads, kTcSmem, s>>>(p, m.err);
   }
 }
