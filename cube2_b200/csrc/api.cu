@@ -45,7 +45,6 @@ struct Plan {
   cufftType type;
   cufftHandle h;
   int pad = 0;   // C2R into the interior of arrays with `pad` ghost points per side
-  int rank = 3;  // 3: whole meshes; 2: the x-y planes of meshes (batch = planes)
 };
 
 struct Ctx {
@@ -226,7 +225,11 @@ static int ensure_device() {
   CU(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
   CU(cudaStreamCreateWithFlags(&g.copy, cudaStreamNonBlocking));
   CU(cudaEventCreateWithFlags(&g.vp_ready, cudaEventDisableTiming));
-  CU(cudaStreamCreateWithFlags(&g.side, cudaStreamNonBlocking));
+  // the binning beside PM3 goes first wherever a block ends: it waits on memory latency and hides in what the
+  // transforms leave, but only if it is resident (512^3 particles: 54.3 ms a kick without, 50.3 with)
+  int least = 0, greatest = 0;
+  CU(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  CU(cudaStreamCreateWithPriority(&g.side, cudaStreamNonBlocking, greatest));
   CU(cudaEventCreateWithFlags(&g.ev_fork, cudaEventDisableTiming));
   CU(cudaEventCreateWithFlags(&g.ev_join, cudaEventDisableTiming));
   for (auto &e : g.ev_tile) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -309,34 +312,10 @@ static int wait_vp() {
   return CUBE_OK;
 }
 
-// Two-dimensional transforms of `batch` consecutive x-y planes of side n: R2C from real planes
-// of n^2 points to half-spectrum planes of n (n/2 + 1); C2R back, into planes of n^2 points or,
-// with pad > 0, into the interior rows of planes of (n + 2 pad)^2 points.
-static int get_plan2d(int n, int batch, cufftType type, int pad, cufftHandle *out) {
-  for (auto &p : g.plans)
-    if (p.rank == 2 && p.n == n && p.batch == batch && p.type == type && p.pad == pad) {
-      CF(cufftSetStream(p.h, g.stream));
-      *out = p.h;
-      return CUBE_OK;
-    }
-  Plan p{n, batch, type, 0, pad, 2};
-  const int h = n / 2 + 1, m = n + 2 * pad;
-  int dims[2] = {n, n}, real[2] = {m, m}, cplx[2] = {n, h};
-  if (type == CUFFT_R2C) {
-    CF(cufftPlanMany(&p.h, 2, dims, real, 1, m * m, cplx, 1, n * h, CUFFT_R2C, batch));
-  } else {
-    CF(cufftPlanMany(&p.h, 2, dims, cplx, 1, n * h, real, 1, m * m, CUFFT_C2R, batch));
-  }
-  CF(cufftSetStream(p.h, g.stream));
-  g.plans.push_back(p);
-  *out = p.h;
-  return CUBE_OK;
-}
-
 // C2R whose output lands in the interior of [batch][(n+2 pad)^3] arrays (advanced layout)
 static int get_plan_padded_c2r(int n, int batch, int pad, cufftHandle *out) {
   for (auto &p : g.plans)
-    if (p.rank == 3 && p.n == n && p.batch == batch && p.type == CUFFT_C2R && p.pad == pad) {
+    if (p.n == n && p.batch == batch && p.type == CUFFT_C2R && p.pad == pad) {
       CF(cufftSetStream(p.h, g.stream));
       *out = p.h;
       return CUBE_OK;
@@ -353,7 +332,7 @@ static int get_plan_padded_c2r(int n, int batch, int pad, cufftHandle *out) {
 
 static int get_plan(int n, int batch, cufftType type, cufftHandle *out) {
   for (auto &p : g.plans)
-    if (p.rank == 3 && p.n == n && p.batch == batch && p.type == type && p.pad == 0) {
+    if (p.n == n && p.batch == batch && p.type == type && p.pad == 0) {
       CF(cufftSetStream(p.h, g.stream));
       *out = p.h;
       return CUBE_OK;
@@ -531,7 +510,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
       if (ratio_sf[m.ires_loc[q] - 1] != rsf) return fail(CUBE_ERR_INVALID);
     const int n = (per_tile ? L.nt * L.rcs : L.ng) * rsf;
     const int nslots = per_tile ? L.ntile : 1;
-    const int64_t n3 = (int64_t)n * n * n, nk = (int64_t)n * n * (n / 2 + 1);
+    const int64_t n3 = (int64_t)n * n * n, nk = pm3_spec_elems(n, nslots);
     float *G = nullptr;
     CK(get_green_periodic(n, rsf, &G));
     CK(grow(g.rho, sizeof(float) * n3 * nslots));
@@ -558,6 +537,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     a.rhok = (cufftComplex *)g.rhok.p;
     a.force = nullptr;
     a.green = G;
+    a.green_sym = true;
     a.mass = mass;
     a.kick = kick;
     a.vp = d.vp;
@@ -585,16 +565,9 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
       a.dep_items = (int2 *)g.dep_items.p;
       a.n_particles_hint = d.n_used;
     }
-    // k-space step: two-dimensional transforms of the x-y planes around the fused z step where
-    // the mesh side allows, otherwise three-dimensional transforms around the Green multiply.
-    // Several padded meshes (one per tile) take the three-dimensional path: their planes are
-    // not equally spaced, and one plane C2R call per mesh costs more than it saves.
-    const bool zsplit = pm3_kspace_z_ok(n) && (!fused || nslots == 1);
-    cufftHandle fw, bw;
-    if (zsplit) {
-      CK(get_plan2d(n, n * nslots, CUFFT_R2C, 0, &fw));
-      CK(get_plan2d(n, fused ? n : n * nslots, CUFFT_C2R, fused ? kPotPad : 0, &bw));
-    } else {
+    const bool own = pm3_fft_ok(n, nslots);
+    cufftHandle fw = 0, bw = 0;
+    if (!own) {
       CK(get_plan(n, nslots, CUFFT_R2C, &fw));
       if (fused) CK(get_plan_padded_c2r(n, nslots, kPotPad, &bw));
       else CK(get_plan(n, nslots, CUFFT_C2R, &bw));
@@ -612,23 +585,24 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     } else {
       g.launches += launch_pm3_deposit(a, g.stream);
     }
-    CF(cufftExecR2C(fw, (cufftReal *)g.rho.p, (cufftComplex *)g.rhok.p));
-    if (zsplit) launch_pm3_kspace_z(a, g.stream);
-    else launch_pm3_kspace(a, g.stream);
-    if (fused) {
-      // the potential into the interior of the padded array, then its periodic ghost points
-      const int64_t mm = n + 2 * kPotPad;
-      float *interior = a.phi + (kPotPad * mm + kPotPad) * mm + kPotPad;
-      if (zsplit) {  // plane transforms, one mesh at a time (the padded meshes are m^3 apart)
-        for (int sl = 0; sl < nslots; sl++)
-          CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p + (int64_t)sl * nk, (cufftReal *)(interior + sl * mm * mm * mm)));
-      } else {
-        CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)interior));
-      }
-      launch_pm3_ghosts(a, g.stream);
+    if (own) {
+      g.launches += launch_pm3_fft(a, g.stream);
     } else {
-      CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)g.rho.p));  // potential
+      CF(cufftExecR2C(fw, (cufftReal *)g.rho.p, (cufftComplex *)g.rhok.p));
+      launch_pm3_kspace(a, g.stream);
+      if (fused) {
+        // the potential into the interior of the padded array, then its periodic ghost points
+        const int64_t mm = n + 2 * kPotPad;
+        CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)(a.phi + (kPotPad * mm + kPotPad) * mm + kPotPad)));
+        launch_pm3_ghosts(a, g.stream);
+      } else {
+        CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)g.rho.p));  // potential
+      }
+      g.launches += fused ? 2 : 1;
+    }
+    if (!fused) {
       launch_pm3_force(a, g.stream);
+      g.launches += 1;
     }
     auto gather = [&](const PM3Args &ga) {
       if (fused) launch_pm3_force_gather(ga, g.stream);
@@ -652,7 +626,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
       CK(wait_vp());
       gather(a);
     }
-    g.launches += 3;  // k-space, then ghosts + force-gather or force + gather
+    g.launches += 1;
     CU(cudaGetLastError());
     return CUBE_OK;
   }
@@ -673,7 +647,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
     if (!gk || !gk[lev - 2]) return fail(CUBE_ERR_INVALID);
     const int rsf = ratio_sf[lev - 1];
     const int nfp = L.ntt * L.rcs * rsf, nfb = L.rcs * rsf, n = nfp + 2 * nfb;
-    const int64_t n3 = (int64_t)n * n * n, nk = (int64_t)n * n * (n / 2 + 1);
+    const int64_t n3 = (int64_t)n * n * n, nk = pm3_spec_elems(n, 1);
     const size_t per_slot = sizeof(float) * (size_t)n3 * 4 + sizeof(cufftComplex) * (size_t)nk;
     const size_t budget = (size_t)8 << 30;
     int bmax = (int)std::max<size_t>(1, budget / per_slot);
@@ -707,7 +681,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
   for (const Batch &bt : batches) {
     const int rsf = ratio_sf[bt.lev - 1], n = bt.n, nj = bt.nj;
     const int nfp = L.ntt * L.rcs * rsf, nfb = L.rcs * rsf;
-    const int64_t n3 = (int64_t)n * n * n, nk = (int64_t)n * n * (n / 2 + 1);
+    const int64_t n3 = (int64_t)n * n * n, nk = pm3_spec_elems(n, 1);
     float *G = nullptr;
     CK(get_green_host(gk[bt.lev - 2], n, &G));
     int nb = nj;
@@ -760,14 +734,21 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
       CK(grow(g.force, sizeof(float) * n3 * 3 * nb));
       a.force = (float *)g.force.p;
     }
-    cufftHandle fw, bw;
-    CK(get_plan(n, nb, CUFFT_R2C, &fw));
-    CK(get_plan(n, nb, CUFFT_C2R, &bw));
+    const bool own = pm3_fft_ok(n, nb);
+    cufftHandle fw = 0, bw = 0;
+    if (!own) {
+      CK(get_plan(n, nb, CUFFT_R2C, &fw));
+      CK(get_plan(n, nb, CUFFT_C2R, &bw));
+    }
     CU(cudaMemsetAsync(g.rho.p, 0, sizeof(float) * n3 * nb, g.stream));
     g.launches += launch_pm3_deposit(a, g.stream);
-    CF(cufftExecR2C(fw, (cufftReal *)g.rho.p, (cufftComplex *)g.rhok.p));
-    launch_pm3_kspace(a, g.stream);
-    CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)g.rho.p));  // potentials
+    if (own) {
+      g.launches += launch_pm3_fft(a, g.stream) - 1;
+    } else {
+      CF(cufftExecR2C(fw, (cufftReal *)g.rho.p, (cufftComplex *)g.rhok.p));
+      launch_pm3_kspace(a, g.stream);
+      CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)g.rho.p));  // potentials
+    }
     if (fused) {
       CK(wait_vp());
       if (!launch_pm3_force_gather(a, g.stream)) return fail(CUBE_ERR_CUDA);
@@ -1446,7 +1427,7 @@ static int run_pm_layer(int layer, const Dev &d, float mass, float kick, float a
   const bool pm1 = layer == 1;
   const int n = pm1 ? L.nc : L.nte * L.rcs;
   const int nslots = pm1 ? 1 : L.ntile;
-  const int64_t n3 = (int64_t)n * n * n, nk = (int64_t)n * n * (n / 2 + 1);
+  const int64_t n3 = (int64_t)n * n * n, nk = pm3_spec_elems(n, nslots);
   CK(stage_begin((size_t)1 << 20));
   CK(grow(g.cell_base, sizeof(int64_t) * (size_t)L.ntile * L.nte * L.nte * L.nte));
   CK(grow(g.out, sizeof(float) * 8));
@@ -1497,19 +1478,27 @@ static int run_pm_layer(int layer, const Dev &d, float mass, float kick, float a
   a.rhok = (cufftComplex *)g.rhok.p;
   a.force = (float *)g.force.p;
   a.green = G;
+  a.green_sym = true;
   a.mass = mass;
   a.kick = kick;
   a.vp = d.vp;
   a.out = (float *)g.out.p;
   a.want_vmax = 1;
-  cufftHandle fw, bw;
-  CK(get_plan(n, nslots, CUFFT_R2C, &fw));
-  CK(get_plan(n, nslots, CUFFT_C2R, &bw));
+  const bool own = pm3_fft_ok(n, nslots);
+  cufftHandle fw = 0, bw = 0;
+  if (!own) {
+    CK(get_plan(n, nslots, CUFFT_R2C, &fw));
+    CK(get_plan(n, nslots, CUFFT_C2R, &bw));
+  }
   CU(cudaMemsetAsync(g.rho.p, 0, sizeof(float) * n3 * nslots, g.stream));
   launch_pm3_deposit(a, g.stream);
-  CF(cufftExecR2C(fw, (cufftReal *)g.rho.p, (cufftComplex *)g.rhok.p));
-  launch_pm3_kspace(a, g.stream);
-  CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)g.rho.p));
+  if (own) {
+    g.launches += launch_pm3_fft(a, g.stream) - 1;
+  } else {
+    CF(cufftExecR2C(fw, (cufftReal *)g.rho.p, (cufftComplex *)g.rhok.p));
+    launch_pm3_kspace(a, g.stream);
+    CF(cufftExecC2R(bw, (cufftComplex *)g.rhok.p, (cufftReal *)g.rho.p));
+  }
   launch_pm3_force(a, g.stream);
   launch_pm3_gather(a, g.stream);
   g.launches += 5;

@@ -249,9 +249,10 @@ struct PM3Args {
   const int32_t *rhoc;
   const int64_t *cell_base;
   float *rho;            // [nslots][n^3] density, then potential
-  cufftComplex *rhok;    // [nslots][n*n*(n/2+1)]
+  cufftComplex *rhok;    // [nslots][pm3_spec_elems]
   float *force;          // [nslots*3][n^3]
   const float *green;    // [n*n*(n/2+1)]
+  bool green_sym = false;  // it is one of this library's: green[k3][k2][k1] = green[n - k3][k2][k1] = green[k3][n - k2][k1]
   float mass, kick;
   float *vp;
   float *out;
@@ -273,10 +274,11 @@ int launch_pm3_deposit(const PM3Args &a, cudaStream_t s);  // returns the kernel
 // CIC instead of TSC on the brick kernels' geometry (pm3_brick_mc != 0, else nothing and 0): cell-centred points
 int launch_cic_bricks(const PM3Args &a, cudaStream_t s);
 void launch_pm3_kspace(const PM3Args &a, cudaStream_t s);
-// the k-space step on the spectrum of two-dimensional x-y transforms: z transform, Green
-// multiply, inverse z transform (mesh sides where pm3_kspace_z_ok)
-bool pm3_kspace_z_ok(int n);
-void launch_pm3_kspace_z(const PM3Args &a, cudaStream_t s);
+// Density to potential in this library's own transforms (mesh sides where pm3_fft_ok): a.rho to a.phi, with
+// ghost points where a.phi_pad > 0, or in place without a.phi.  Returns the kernels it launched
+bool pm3_fft_ok(int n, int nslots);
+int launch_pm3_fft(const PM3Args &a, cudaStream_t s);
+int64_t pm3_spec_elems(int n, int nslots);  // complex values of a.rhok a slot
 void launch_pm3_force(const PM3Args &a, cudaStream_t s);  // force arrays + f2max from the potential
 void launch_pm3_gather(const PM3Args &a, cudaStream_t s);
 // the force difference fused into the gather, brick by brick (no force arrays); returns false
