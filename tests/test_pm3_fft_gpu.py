@@ -36,7 +36,9 @@ def _truth(pos, ng, n, G):
     return F.cpu().numpy(), float(phi.pow(2).mean().sqrt())
 
 
-@pytest.mark.parametrize("n,nnt", [(64, 1), (128, 2), (256, 1), (512, 2), (1024, 2)])
+@pytest.mark.parametrize("n,nnt", [(64, 1), (80, 1), (96, 2), (128, 2), (144, 3), (160, 2), (192, 2), (240, 2), (256, 1),
+                                   (288, 2), (320, 1), (384, 2), (480, 2), (512, 2), (576, 2), (640, 2), (768, 2),
+                                   (960, 2), (1024, 2)])
 def test_transforms_of_every_side(gpu, n, nnt):
     from cube2_b200.kick import CUBE_PM3_PERIODIC, FineKick, green_table
     from cube2_b200.layout import RATIO_SF, Layout, build_image, ixyz3_table
