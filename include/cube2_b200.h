@@ -256,10 +256,11 @@ int cube_kick_sums(const int32_t *d_rhoc, const int64_t *d_idx_b_r, int64_t n_us
 
 /* The PP force kernel comes in several shapes: `chunk` i-particles per work item (a
  * crowded PP cell of n particles is split into ceil(n / chunk) items, one warp each),
- * `jtile` candidates a warp stages in shared memory between flushes, the pair loop
+ * `jtile` candidates a warp stages in shared memory between flushes, the inner loop
  * unrolled `unroll` times, registers budgeted for `blocks` resident blocks per SM, and
- * `packed` = 1 for the pair law on packed f32x2 arithmetic (two candidates per lane and
- * instruction; each pair's force is the scalar one bit for bit).  By
+ * `packed` = 1 for the kernel that lists the pairs within range on the tensor cores and
+ * evaluates only those, two at a time in packed f32x2 arithmetic (each pair's force is the
+ * scalar one bit for bit), 0 for the one that evaluates every staged candidate.  By
  * default the first PP kick of each (layout, per-tile PP grids, PP ranges, octave of
  * n_used) times every shape on its own particles (work list + force kernel, into scratch
  * velocities; the host waits for it once) and that key keeps the fastest; a kick being
