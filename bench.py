@@ -325,7 +325,7 @@ def run_ours(args, rank, world, local_rank):
     ppf_ms = float(np.mean(stages[:, 2])) if len(stages) else None
     flops = PP_FLOP_PER_PAIR * pairs
     achieved = flops / (ppf_ms * 1e-3) / 1e12 if ppf_ms else None
-    roofline = {"kernel": "k_pp_force (PP pair force + kick)", "bound": "fp32", "achieved": achieved,
+    roofline = {"kernel": "k_pp_pairs (PP pair force + kick)", "bound": "fp32", "achieved": achieved,
                 "peak": fp32_peak, "unit": "TFLOP/s", "frac": (achieved / fp32_peak) if achieved else None,
                 "peak_source": "FP32 FMA probe measured in this run (MEASURED_PEAKS.json has no FP32 figure)",
                 "flops_per_launch": int(flops), "pairs_per_launch": int(pairs),
