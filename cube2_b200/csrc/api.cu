@@ -95,8 +95,10 @@ struct Ctx {
   // What a kick starts from zero, cleared by one memset: the outputs and status word (out), the binning's
   // counters, the brick kernels' counters and the PP schedule, at the offsets below
   Buf out;
-  // learned shell: positions of the copies, fine-grid CIC density, listed copies, stencil rows of the density
-  Buf mlp_pos, mlp_rho, mlp_n, mlp_tab;
+  // learned shell: positions of the copies, fine-grid CIC density, listed copies, stencil rows of the density, and
+  // the density's own mesh jobs and deposit work list.  The kick's (jobs, dep_items) hold another mesh's offsets and
+  // bricks: a kick may still be running on another stream
+  Buf mlp_pos, mlp_rho, mlp_n, mlp_tab, mlp_jobs, mlp_items;
   // PP kernel shape: fixed (pp_fixed >= 0, cube_pp_set_shape) or autotuned, keyed by
   // pp_shape_key; pp_ms holds the last tuning's times, pp_last the shape of the last PP kick
   int pp_fixed = -1;
@@ -1961,14 +1963,14 @@ static int mlp_density(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const in
   CK(grow(g.mlp_pos, sizeof(float4) * (size_t)std::max<int64_t>(n_used, 1)));
   CK(grow(g.mlp_rho, sizeof(float) * (size_t)ng3));
   CK(grow(g.mlp_n, sizeof(unsigned long long)));
-  CK(grow(g.jobs, sizeof(MeshJob) * (size_t)L.ntile));
-  launch_cell_table_jobs(L, d_rhoc, d_idx_b_r, (int64_t *)g.cell_base.p, (double)L.rcs, false, (MeshJob *)g.jobs.p, s);
+  CK(grow(g.mlp_jobs, sizeof(MeshJob) * (size_t)L.ntile));
+  launch_cell_table_jobs(L, d_rhoc, d_idx_b_r, (int64_t *)g.cell_base.p, (double)L.rcs, false, (MeshJob *)g.mlp_jobs.p, s);
   CU(cudaMemsetAsync(g.mlp_rho.p, 0, sizeof(float) * ng3, s));
   PM3Args a{};  // the fine grid as a mesh of ratio_cs points per coarse cell
   a.L = &g.L;
   a.n = L.ng;
   a.nslots = 1;
-  a.jobs = (const MeshJob *)g.jobs.p;
+  a.jobs = (const MeshJob *)g.mlp_jobs.p;
   a.njobs = L.ntile;
   for (int q = 0; q < 3; q++) a.rdep[q] = a.ract[q] = L.nt;
   a.wrap = 1;
@@ -1978,8 +1980,8 @@ static int mlp_density(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const in
   a.cell_base = (const int64_t *)g.cell_base.p;
   a.rho = (float *)g.mlp_rho.p;
   a.num_sms = g.num_sms;
-  CK(grow(g.dep_items, pm3_dep_items_bytes((int64_t)L.nt * L.nt * L.nt, L.ntile, n_used)));
-  a.dep_items = (int2 *)g.dep_items.p;
+  CK(grow(g.mlp_items, pm3_dep_items_bytes((int64_t)L.nt * L.nt * L.nt, L.ntile, n_used)));
+  a.dep_items = (int2 *)g.mlp_items.p;
   a.n_particles_hint = n_used;
   const bool bricks = pm3_brick_mc(a) > 0;
   if (list || !bricks) {
@@ -2218,6 +2220,8 @@ void c_pm3_fft_finalize(void) {
   release(g.mlp_rho);
   release(g.mlp_n);
   release(g.mlp_tab);
+  release(g.mlp_jobs);
+  release(g.mlp_items);
 }
 
 void c_gpu_velocity_finalize(void) {
