@@ -428,10 +428,11 @@ static void fill_ptotal(const Meta &m, const int32_t *rhoc, double *ptotal) {
 // then the brick kernels' counters (a pair for each of kBrickCtrs launches), then the PP schedule.
 constexpr int kOutErr = 5, kOutCtr = 8, kOutBrick = kOutCtr + 128, kBrickCtrs = 64, kOutSched = kOutBrick + 2 * kBrickCtrs;
 static int32_t *out_word(int w) { return (int32_t *)g.out.p + w; }
-static int clear_outputs(cudaStream_t s) {
+// `pp`: the PP schedule too; without PP it stays the last PP kick's, which cube_pp_work_stats reads
+static int clear_outputs(bool pp, cudaStream_t s) {
   const size_t bytes = sizeof(int32_t) * (kOutSched + sched_ints(g.L.ntile));
   CK(grow(g.out, bytes));
-  CU(cudaMemsetAsync(g.out.p, 0, bytes, s));
+  CU(cudaMemsetAsync(g.out.p, 0, pp ? bytes : sizeof(int32_t) * kOutSched, s));
   return CUBE_OK;
 }
 
@@ -1013,7 +1014,7 @@ static int run_kick(const int32_t *ires, const int32_t *ixyz3, const int32_t *ra
   size_t soff = 0;
   // kick coefficient a_mid*dt/6/pi (kick.f90:529, pp_force_kernel.c:355)
   const float kick = (float)((double)(a_mid * dt / 6.0f) / 3.14159265358979323846);
-  CK(clear_outputs(g.stream));
+  CK(clear_outputs(do_pp, g.stream));
   if (g.timing) {
     g.ring_cur = g.ring_next;
     g.ring_next = (g.ring_next + 1) % Ctx::kRing;
@@ -2369,7 +2370,7 @@ int cube_pp_pair_count(const int32_t *ires, const int32_t *ixyz3, const float *a
   CU(cudaMemcpyAsync(g.rhoc.p, rhoc, sizeof(int32_t) * nrows * L.nte, cudaMemcpyHostToDevice, g.stream));
   CU(cudaMemcpyAsync(g.idx.p, idx_b_r, sizeof(int64_t) * nrows, cudaMemcpyHostToDevice, g.stream));
   if (n_used) CU(cudaMemcpyAsync(g.xp.p, xp, sizeof(int16_t) * 3 * n_used, cudaMemcpyHostToDevice, g.stream));
-  CK(clear_outputs(g.stream));
+  CK(clear_outputs(true, g.stream));
   launch_cell_table(L, (const int32_t *)g.rhoc.p, (const int64_t *)g.idx.p, (int64_t *)g.cell_base.p, g.stream);
   Dev d{(const int16_t *)g.xp.p, (const int32_t *)g.rhoc.p, (const int64_t *)g.idx.p, nullptr, n_used};
   size_t soff = 0;
