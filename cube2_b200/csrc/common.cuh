@@ -117,13 +117,18 @@ __device__ __forceinline__ unsigned long long ns_now() {
   return t;
 }
 constexpr unsigned long long kBulkWaitNs = 1000000000ull;  // bound of one wait for a brick's copies: 1 s
-// wait for a phase of the mbarrier, at most kBulkWaitNs; false when the wait gave up
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
+// Wait for a phase of the mbarrier, at most `limit` ns; false when the wait gave up.  Called by whole warps, and all
+// lanes get the same answer: each reads its own clock, and at the limit one lane may see the phase complete that
+// another has given up.  Were they to part there, the warp would hang in its next full-mask instruction.
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, unsigned long long limit = kBulkWaitNs) {
+  bool done = mbar_try_wait(bar, parity);
+  if (__all_sync(0xffffffffu, done)) return true;
   const unsigned long long t0 = ns_now();
-  while (!mbar_try_wait(bar, parity))
-    if (ns_now() - t0 > kBulkWaitNs) return false;
-  return true;
+  do {
+    done = done || mbar_try_wait(bar, parity);
+    if (__all_sync(0xffffffffu, done)) return true;
+  } while (!__any_sync(0xffffffffu, ns_now() - t0 > limit));
+  return false;
 }
 // bulk asynchronous copy global -> this CTA's shared memory, completing on the mbarrier
 // (both addresses 16-byte aligned, bytes a multiple of 16)

@@ -476,7 +476,8 @@ __device__ __forceinline__ int64_t brick_particle(int k, const BrickRows &br, co
 //   consumers: every active particle of the brick gathers its 27 TSC points from the force
 //     buffer and is kicked (kick.f90:497-540).  A thread's next particle, of this brick or the next, is
 //     loaded (offset and velocity) before the current one is worked on.
-// The buffers change hands through mbarriers, every wait bounded.  The arithmetic (weights, products,
+// The buffers change hands through mbarriers, every wait bounded and decided by whole warps (the roles are whole
+// warps): one that gives up leaves for the block's last barrier, the others' next waits run out and they follow.  The arithmetic (weights, products,
 // summation order) is the one of k_force_zm followed by k_gather, and the force arrays never reach HBM.
 //
 // Before the scheduler and the prefetch (the producers claimed the bricks, the consumers met each brick's
