@@ -1487,6 +1487,11 @@ static int run_pm_layer(int layer, const Dev &d, float mass, float kick, float a
   a.vp = d.vp;
   a.out = (float *)g.out.p;
   a.want_vmax = 1;
+  // Crowded bricks in pieces, as in the kick: without the list one block walks a brick however many particles it
+  // holds, and its fixed-point scale falls with their number (2^16 at 10^5)
+  CK(grow(g.dep_items, pm3_dep_items_bytes((int64_t)a.rdep[0] * a.rdep[1] * a.rdep[2], a.njobs, d.n_used)));
+  a.dep_items = (int2 *)g.dep_items.p;
+  a.n_particles_hint = d.n_used;
   const bool own = pm3_fft_ok(n, nslots);
   cufftHandle fw = 0, bw = 0;
   if (!own) {
@@ -1494,7 +1499,7 @@ static int run_pm_layer(int layer, const Dev &d, float mass, float kick, float a
     CK(get_plan(n, nslots, CUFFT_C2R, &bw));
   }
   CU(cudaMemsetAsync(g.rho.p, 0, sizeof(float) * n3 * nslots, g.stream));
-  launch_pm3_deposit(a, g.stream);
+  g.launches += launch_pm3_deposit(a, g.stream);
   if (own) {
     g.launches += launch_pm3_fft(a, g.stream) - 1;
   } else {
@@ -1504,7 +1509,7 @@ static int run_pm_layer(int layer, const Dev &d, float mass, float kick, float a
   }
   launch_pm3_force(a, g.stream);
   launch_pm3_gather(a, g.stream);
-  g.launches += 5;
+  g.launches += 4;
   CU(cudaGetLastError());
   CK(stage_end());
   CU(cudaMemcpyAsync(out, g.out.p, sizeof(float) * 5, cudaMemcpyDeviceToHost, g.stream));

@@ -839,9 +839,12 @@ constexpr int kAccW = kBrick + 2;  // y, z window owned - 1 .. owned + kBrick
 
 constexpr int kDepChunk = 2048;  // particles of one deposit work item (a crowded brick makes several)
 
-// The deposit's work list: every brick with particles makes ceil(particles / kDepChunk) items
-// (brick, chunk, chunks), so a crowded brick is spread over several blocks whose windows add up
-// in the mesh; empty bricks make none.  One thread per brick; items[0..count) in any order.
+// The deposit's work list: brick b's item (brick, chunk, chunks) at items[b], no chunks where it has no particles.  A
+// brick of more than `chunk` particles makes ceil(particles / chunk) items, the others behind the nbricks first ones in
+// any order, so a crowded brick is spread over several blocks whose windows add up in the mesh.  One thread
+// per brick; *count counts the items behind.  They fit unless the cells hold more particles than the list was
+// sized for (the counts or the particle number are wrong): then an error and no item where a status word is given,
+// else one item.
 __global__ void k_dep_items(PM3K p, int mc, int64_t nbricks, int chunk, int2 *items, int *count, int64_t cap) {
   const int cb = kBrick / mc;
   for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nbricks;
@@ -854,19 +857,22 @@ __global__ void k_dep_items(PM3K p, int mc, int64_t nbricks, int chunk, int2 *it
         const int32_t *r = p.rhoc + ((t * p.nte + q.ck0 + k) * p.nte + q.cj0 + j) * p.nte + q.ci0;
         for (int i = 0; i < q.n[0]; i++) total += r[i];
       }
-    if (total == 0) continue;
-    const int nch = min((total + chunk - 1) / chunk, 0x7fff);
-    const int at = atomicAdd(count, nch);
-    if (at + nch > cap) {  // more particles in the cells than stored: the cell counts are wrong
-      if (p.err) atomicOr(p.err, 1 << CUBE_ERR_CAPACITY);
-      continue;
+    int nch = min((total + chunk - 1) / chunk, 0x7fff);
+    if (nch > 1) {
+      const int64_t at = nbricks + atomicAdd(count, nch - 1);
+      if (at + nch - 1 > cap) {
+        if (p.err) atomicOr(p.err, 1 << CUBE_ERR_CAPACITY);
+        for (int64_t i = at; i < cap; i++) items[i] = make_int2(0, 0);
+        nch = p.err ? 0 : 1;
+      }
+      for (int c = 1; c < nch; c++) items[at + c - 1] = make_int2((int)b, c | (nch << 16));
     }
-    for (int c = 0; c < nch; c++) items[at + c] = make_int2((int)b, c | (nch << 16));
+    items[b] = make_int2((int)b, nch << 16);
   }
 }
 
 template <bool CIC>
-__global__ void __launch_bounds__(kDepThreads, kDepBlocks) k_deposit_brick(PM3K p, int mc, const int2 *items,
+__global__ void __launch_bounds__(kDepThreads, kDepBlocks) k_deposit_brick(PM3K p, int mc, int64_t nbricks, const int2 *items,
                                                                                const int *count) {
   __shared__ __align__(16) unsigned acc[kAccW * kAccW * kAccX];
   __shared__ int64_t rbase[kMaxRowsPerBrick];
@@ -874,10 +880,11 @@ __global__ void __launch_bounds__(kDepThreads, kDepBlocks) k_deposit_brick(PM3K 
   __shared__ int rcell[kMaxRowsPerBrick * (kMaxCb + 1)];
   int2 item = make_int2((int)blockIdx.x, 1 << 16);  // without a work list: a whole brick
   if (items) {
-    if ((int)blockIdx.x >= min(*count, (int)gridDim.x)) return;
+    if (blockIdx.x >= nbricks && blockIdx.x - nbricks >= *count) return;
     item = items[blockIdx.x];
   }
   const int chunk = item.y & 0xffff, nch = item.y >> 16;
+  if (nch == 0) return;
   const int cb = kBrick / mc;
   const BrickPos q = brick_pos(p, item.x, cb, p.rdep, p.rdep);
   const MeshJob &J = p.jobs[q.j];
@@ -981,34 +988,43 @@ void set_smem_attr_once(const void *fn, size_t bytes) {
 }
 
 size_t pm3_dep_items_bytes(int64_t cells_per_job, int njobs, int64_t n_used) {
-  // bricks hold at least one coarse cell: one item per cell, plus one per kDepChunk particles, plus the count
+  // bricks hold at least one coarse cell: one item per cell at most, plus one per kDepChunk particles, plus the count
   return sizeof(int2) * ((size_t)cells_per_job * njobs + (size_t)(n_used / kDepChunk) + 2);
+}
+
+int64_t pm3_deposit_bricks(const PM3Args &a) {
+  const int mc = pm3_brick_mc(a);
+  if (!mc) return 0;
+  const int cb = kBrick / mc;
+  return (int64_t)bricks_of(a.rdep[0], cb) * bricks_of(a.rdep[1], cb) * bricks_of(a.rdep[2], cb) * a.njobs;
 }
 
 // the brick deposit (TSC or CIC), with its work list where the caller gives the scratch for one
 template <bool CIC>
 static int launch_deposit_bricks(const PM3Args &a, int mc, cudaStream_t s) {
   const PM3K p = make_k(a);
-  const int cb = kBrick / mc;
-  const int64_t nbricks = (int64_t)bricks_of(a.rdep[0], cb) * bricks_of(a.rdep[1], cb) * bricks_of(a.rdep[2], cb) * a.njobs;
+  const int64_t nbricks = pm3_deposit_bricks(a);
   if (nbricks <= 0) return 0;
   if (!a.dep_items) {
-    k_deposit_brick<CIC><<<(unsigned)nbricks, kDepThreads, 0, s>>>(p, mc, nullptr, nullptr);
+    k_deposit_brick<CIC><<<(unsigned)nbricks, kDepThreads, 0, s>>>(p, mc, nbricks, nullptr, nullptr);
     return 1;
   }
-  // at most one item per brick plus one per kDepChunk particles
+  // one item per brick, and behind them at most one per kDepChunk particles
   const int64_t cap = nbricks + a.n_particles_hint / kDepChunk + 1;
   int *count = a.dep_count ? a.dep_count : reinterpret_cast<int *>(a.dep_items + cap);
   if (!a.dep_count || !a.zeroed) cudaMemsetAsync(count, 0, sizeof(int), s);
   k_dep_items<<<(unsigned)std::min<int64_t>((nbricks + 255) / 256, 4096), 256, 0, s>>>(p, mc, nbricks, kDepChunk,
                                                                                      a.dep_items, count, cap);
   // one block per possible item: resident blocks that loop over the list took 6 % longer (barriers, fixed shares)
-  k_deposit_brick<CIC><<<(unsigned)cap, kDepThreads, 0, s>>>(p, mc, a.dep_items, count);
+  k_deposit_brick<CIC><<<(unsigned)cap, kDepThreads, 0, s>>>(p, mc, nbricks, a.dep_items, count);
   return 2;
 }
 
 int launch_pm3_deposit(const PM3Args &a, cudaStream_t s) {
-  if (const int mc = pm3_brick_mc(a)) return launch_deposit_bricks<false>(a, mc, s);
+  // Buffered meshes of fewer bricks than multiprocessors go by coarse cell, a warp each: the tile mesh of PM2 on a 32^3
+  // box (27 bricks of a 40^3 mesh) takes 113 us a call so, 121 by bricks; eight of them (216 bricks) 176 and 146
+  const int mc = pm3_brick_mc(a);
+  if (mc && (a.wrap || pm3_deposit_bricks(a) >= a.num_sms)) return launch_deposit_bricks<false>(a, mc, s);
   const PM3K p = make_k(a);
   const int64_t warps = (int64_t)a.rdep[0] * a.rdep[1] * a.rdep[2] * a.njobs;
   k_deposit<<<(unsigned)((warps + kWarps - 1) / kWarps), kWarps * 32, 0, s>>>(p);
