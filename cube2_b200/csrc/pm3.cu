@@ -830,8 +830,10 @@ void launch_pm3_force(const PM3Args &a, cudaStream_t s) {
 // one 16-byte vector reduction per group of four points that received anything: every mesh point
 // takes at most one global reduction per brick that reaches it, instead of one per particle.
 // kick.f90:420-468 sums the same weights; the integer sums make the brick's part exact and
-// independent of the order of the atomics (the rounding of a weight to 2^-e, e >= 15 for
-// bricks of up to 10^5 particles, is far below the FP32 rounding of the density).
+// independent of the order of the atomics.  An item has at most kDepChunk particles (unless its brick has 6e7), so
+// TSC weights are rounded to 2^-22 or finer.  The learned shell's CIC density, up to 4096 particles a uniform brick,
+// starts at the scale of its mean density instead, 2^-26 in a uniform box.  At 2^-20, from the number alone, ten times as
+// many of the network's BF16 inputs differed from the exact density's as with sums in FP32.
 constexpr int kDepThreads = 256;
 constexpr int kDepBlocks = 5;  // resident blocks per SM (48 registers a thread)
 constexpr int kAccX = kBrick + 8;  // x window owned - 4 .. owned + kBrick + 3: whole float4 groups
@@ -878,6 +880,8 @@ __global__ void __launch_bounds__(kDepThreads, kDepBlocks) k_deposit_brick(PM3K 
   __shared__ int64_t rbase[kMaxRowsPerBrick];
   __shared__ int rstart[kMaxRowsPerBrick + 1];
   __shared__ int rcell[kMaxRowsPerBrick * (kMaxCb + 1)];
+  __shared__ unsigned long long s_sum;
+  if (CIC && threadIdx.x == 0) s_sum = 0;
   int2 item = make_int2((int)blockIdx.x, 1 << 16);  // without a work list: a whole brick
   if (items) {
     if (blockIdx.x >= nbricks && blockIdx.x - nbricks >= *count) return;
@@ -895,46 +899,78 @@ __global__ void __launch_bounds__(kDepThreads, kDepBlocks) k_deposit_brick(PM3K 
   // this item's particles of the brick
   const int k0 = (int)((int64_t)br.total * chunk / nch), k1 = (int)((int64_t)br.total * (chunk + 1) / nch);
   if (k1 <= k0) return;
-  // fixed-point scale 2^e: particles * (largest weight) * 2^e < 2^32
-  int e = 24;
-  while (e > 1 && (double)(k1 - k0) * (CIC ? 1.0 : 0.421875) * (double)(1u << e) >= 4294967040.0) e--;
-  const float fs = (float)(1u << e), inv = 1.0f / fs;
-  for (int k = k0 + threadIdx.x; k < k1; k += kDepThreads) {
-    int di, dj, dk;
-    const int64_t ip = brick_particle(k, br, rbase, rstart, rcell, di, dj, dk);
-    const int16_t *qp = p.xp + 3 * ip;
-    if constexpr (CIC) {  // points at cell centres: the first is floor(x - 1/2), from -1 of the brick on
-      float fx, fy, fz;
-      const int lx = cic_brick(di, qp[0], mc, fx) + 4, ly = cic_brick(dj, qp[1], mc, fy) + 1,
-                lz = cic_brick(dk, qp[2], mc, fz) + 1;
-      const float sx[2] = {(1.0f - fx) * fs, fx * fs}, sy[2] = {1.0f - fy, fy}, sz[2] = {1.0f - fz, fz};
+  // Fixed-point scale 2^e: particles * (largest weight) * 2^e < 2^32.  For CIC a point may get 31 times the mean density
+  // plus 31, and if one then gets more, the item is done again with a coarser scale: the sums are exact, so
+  // those of the window tell (each point that has wrapped is 2^32 short)
+  auto fits = [](double most, int e) { return most * (double)(1u << e) < 4294967040.0; };
+  const double most = (double)(k1 - k0) * (CIC ? 1.0 : 0.421875);
+  int e = CIC ? 28 : 24;
+  if constexpr (CIC) {
+    const double points = (double)(q.n[0] * q.n[1] * q.n[2]) * (mc * mc * mc);
+    while (e > 1 && !fits(fmin(most, 31.0 * (1.0 + (double)br.total / points)), e)) e--;
+  } else {
+    while (e > 1 && !fits(most, e)) e--;
+  }
+  const auto deposit = [&](const float fs) {
+    for (int k = k0 + threadIdx.x; k < k1; k += kDepThreads) {
+      int di, dj, dk;
+      const int64_t ip = brick_particle(k, br, rbase, rstart, rcell, di, dj, dk);
+      const int16_t *qp = p.xp + 3 * ip;
+      if constexpr (CIC) {  // points at cell centres: the first is floor(x - 1/2), from -1 of the brick on
+        float fx, fy, fz;
+        const int lx = cic_brick(di, qp[0], mc, fx) + 4, ly = cic_brick(dj, qp[1], mc, fy) + 1,
+                  lz = cic_brick(dk, qp[2], mc, fz) + 1;
+        const float sx[2] = {(1.0f - fx) * fs, fx * fs}, sy[2] = {1.0f - fy, fy}, sz[2] = {1.0f - fz, fz};
 #pragma unroll
-      for (int c = 0; c < 2; c++)
+        for (int c = 0; c < 2; c++)
 #pragma unroll
-        for (int bb = 0; bb < 2; bb++) {
+          for (int bb = 0; bb < 2; bb++) {
+            unsigned *row = acc + ((lz + c) * kAccW + (ly + bb)) * kAccX + lx;
+            atomicAdd(row + 0, __float2uint_rn(sx[0] * sy[bb] * sz[c]));
+            atomicAdd(row + 1, __float2uint_rn(sx[1] * sy[bb] * sz[c]));
+          }
+        continue;
+      }
+      float wx[3], wy[3], wz[3];
+      // window indices of the stencil's first point: x (ix - 1) - (X0 - 4), y (iy - 1) - (Y0 - 1)
+      const int lx = tsc_brick(di, qp[0], mc, wx) + 3, ly = tsc_brick(dj, qp[1], mc, wy), lz = tsc_brick(dk, qp[2], mc, wz);
+      const float sx0 = wx[0] * fs, sx1 = wx[1] * fs, sx2 = wx[2] * fs;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+#pragma unroll
+        for (int bb = 0; bb < 3; bb++) {
           unsigned *row = acc + ((lz + c) * kAccW + (ly + bb)) * kAccX + lx;
-          atomicAdd(row + 0, __float2uint_rn(sx[0] * sy[bb] * sz[c]));
-          atomicAdd(row + 1, __float2uint_rn(sx[1] * sy[bb] * sz[c]));
+          const float yz = wy[bb] * wz[c];
+          atomicAdd(row + 0, __float2uint_rn(sx0 * yz));
+          atomicAdd(row + 1, __float2uint_rn(sx1 * yz));
+          atomicAdd(row + 2, __float2uint_rn(sx2 * yz));
         }
-      continue;
-    }
-    float wx[3], wy[3], wz[3];
-    // window indices of the stencil's first point: x (ix - 1) - (X0 - 4), y (iy - 1) - (Y0 - 1)
-    const int lx = tsc_brick(di, qp[0], mc, wx) + 3, ly = tsc_brick(dj, qp[1], mc, wy), lz = tsc_brick(dk, qp[2], mc, wz);
-    const float sx0 = wx[0] * fs, sx1 = wx[1] * fs, sx2 = wx[2] * fs;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-#pragma unroll
-      for (int bb = 0; bb < 3; bb++) {
-        unsigned *row = acc + ((lz + c) * kAccW + (ly + bb)) * kAccX + lx;
-        const float yz = wy[bb] * wz[c];
-        atomicAdd(row + 0, __float2uint_rn(sx0 * yz));
-        atomicAdd(row + 1, __float2uint_rn(sx1 * yz));
-        atomicAdd(row + 2, __float2uint_rn(sx2 * yz));
       }
     }
-  }
+  };
+  deposit((float)(1u << e));
   __syncthreads();
+  if constexpr (CIC) {
+    while (e > 1 && !fits(most, e)) {  // the same for the whole block
+      unsigned long long sum = 0;
+      for (int e4 = threadIdx.x; e4 < kAccW * kAccW * kAccX / 4; e4 += kDepThreads) {
+        const uint4 u = reinterpret_cast<const uint4 *>(acc)[e4];
+        sum += (unsigned long long)u.x + u.y + u.z + u.w;
+      }
+      for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum, sum);
+      __syncthreads();
+      if (((unsigned long long)(k1 - k0) << e) <= s_sum + 0x80000000ull) break;
+      for (int e4 = threadIdx.x; e4 < kAccW * kAccW * kAccX / 4; e4 += kDepThreads)
+        reinterpret_cast<uint4 *>(acc)[e4] = make_uint4(0u, 0u, 0u, 0u);
+      __syncthreads();
+      if (threadIdx.x == 0) s_sum = 0;  // added to again only behind the next barrier
+      e = max(e - 2, 1);
+      deposit((float)(1u << e));
+      __syncthreads();
+    }
+  }
+  const float inv = 1.0f / (float)(1u << e);
   // Flush: lane (w, xg) of a warp takes x group xg (lane % 6) of window rows 5 pass + w (w < 5), so
   // the group's mesh x index is worked out once and each row's once per pass.
   float *R = p.rho + (int64_t)J.slot * p.n3;
