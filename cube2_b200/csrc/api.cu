@@ -1989,7 +1989,8 @@ static int mlp_density(const int32_t *d_rhoc, const int64_t *d_idx_b_r, const in
   CK(grow(g.mlp_items, pm3_dep_items_bytes((int64_t)L.nt * L.nt * L.nt, L.ntile, n_used)));
   a.dep_items = (int2 *)g.mlp_items.p;
   a.n_particles_hint = n_used;
-  const bool bricks = pm3_brick_mc(a) > 0;
+  // few bricks leave the device idle: by particle then, as where there are none
+  const bool bricks = pm3_deposit_bricks(a) >= g.num_sms;
   if (list || !bricks) {
     launch_mlp_list(L, d_xp, d_rhoc, (const int64_t *)g.cell_base.p, (float4 *)g.mlp_pos.p,
                     (unsigned long long *)g.mlp_n.p, s);
