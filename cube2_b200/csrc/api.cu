@@ -121,7 +121,7 @@ struct Ctx {
   cudaEvent_t tune_ev[2 * kMaxPPShapes] = {};
   void *h_stage = nullptr;  // pinned staging for small tables
   size_t h_stage_cap = 0;
-  float *h_out = nullptr;   // pinned [8]: out[5], err
+  float *h_out = nullptr;   // pinned [8]: out[5], err; [7] a network's training status
   std::vector<GreenEntry> greens;
   std::vector<HostGreen> hgreens;
   std::vector<Plan> plans;
@@ -1919,8 +1919,8 @@ int cube_mlp_create(const float *params, int32_t batch_cap, cube_mlp **out) {
   al(&p.dz, sizeof(float) * B * W);
   al(&p.da, sizeof(float) * B * W);
   al(&p.b4pad, sizeof(float) * kMlpOutPad);
-  al(&p.err, sizeof(int32_t));
-  if (ok) ok = cudaMemset(p.err, 0, sizeof(int32_t)) == cudaSuccess;
+  al(&p.err, 2 * sizeof(int32_t));
+  if (ok) ok = cudaMemset(p.err, 0, 2 * sizeof(int32_t)) == cudaSuccess;
   if (ok) ok = cudaMemcpy(p.master, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice) == cudaSuccess;
   if (ok) ok = cudaMemset(p.mom, 0, sizeof(float) * kMlpParams) == cudaSuccess &&
                cudaMemset(p.vel, 0, sizeof(float) * kMlpParams) == cudaSuccess &&
@@ -1953,8 +1953,13 @@ int cube_mlp_get_params(cube_mlp *h, float *params, float *grads) {
   if (!h || (!params && !grads)) return fail(CUBE_ERR_INVALID);
   CU(cudaSetDevice(h->p.device));
   CU(cudaDeviceSynchronize());
+  // the status of the training steps so far travels ahead of the parameters (pinned word, same stream)
+  CU(cudaMemcpyAsync(&g.h_out[7], h->p.err + kMlpErrTrain, sizeof(int32_t), cudaMemcpyDeviceToHost, nullptr));
   if (params) CU(cudaMemcpy(params, h->p.master, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost));
   if (grads) CU(cudaMemcpy(grads, h->p.grad, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost));
+  int32_t e;
+  memcpy(&e, &g.h_out[7], sizeof(e));
+  if (e) return fail(CUBE_ERR_TIMEOUT);
   return CUBE_OK;
 }
 
@@ -2073,11 +2078,11 @@ int cube_mlp_kick(cube_mlp *h, const int32_t *d_rhoc, const int64_t *d_idx_b_r, 
                    g.mlp_tab.p, g.L.ng, d_vp, kick * scale, g.num_sms, s);
   g.launches += 2;
   CU(cudaGetLastError());
-  // the inference kernel's bounded waits report through a status word: read it once the kick is done
-  int32_t e = 0;
-  CU(cudaMemcpyAsync(&e, h->p.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  // bounded waits (the inference kernel's, and earlier training steps') report through status words: read once the kick is done
+  int32_t e[2] = {0, 0};
+  CU(cudaMemcpyAsync(e, h->p.err, sizeof(e), cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
-  if (e) return fail(CUBE_ERR_TIMEOUT);
+  if (e[0] | e[1]) return fail(CUBE_ERR_TIMEOUT);
   return CUBE_OK;
 }
 

@@ -385,6 +385,7 @@ constexpr int kMlpGradBias = (kMlpParams + 1) / 2 * 2;
 constexpr size_t kMlpGradBytes = sizeof(float) * kMlpGradBias + sizeof(double) * (3 * kMlpW + kMlpOut);
 constexpr int kMlpWbElems = mlp_wboff(3) + kMlpOutPad * kMlpW;
 
+constexpr int kMlpErrTrain = 1;
 struct MlpParams {
   float *master = nullptr, *grad = nullptr, *mom = nullptr, *vel = nullptr;  // [kMlpParams]
   __nv_bfloat16 *wb = nullptr, *wt = nullptr;                                // [kMlpWbElems]
@@ -394,7 +395,7 @@ struct MlpParams {
   __nv_bfloat16 *xb = nullptr, *a[3] = {}, *dyb = nullptr, *dzb = nullptr, *dzt = nullptr, *at = nullptr;
   float *tb = nullptr, *z[3] = {}, *y = nullptr, *dy = nullptr, *dz = nullptr, *da = nullptr, *b4pad = nullptr;
   int device = -1;
-  int32_t *err = nullptr;  // device status word of the inference kernel (bit CUBE_ERR_TIMEOUT)
+  int32_t *err = nullptr;  // device status words (bit CUBE_ERR_TIMEOUT): of inference, and of training at kMlpErrTrain
 };
 void launch_mlp_pos(const Lay &L, const int16_t *xp, const int32_t *rhoc, const int64_t *cell_base, float4 *pos,
                     cudaStream_t s);

@@ -1299,21 +1299,24 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(MlpTrainK p) {
   }
 }
 
-// Adam on the FP32 master parameters (bias gradients arrive in FP64), and the BF16 weight copies
+// Adam on the FP32 master parameters (bias gradients arrive in FP64), and the BF16 weight copies.  Nothing changes
+// once a training step's wait has run out (*err): its gradients are not whole.
 __global__ void k_adam_pack(float *w, float *grad, const double *gbias, float *m, float *v, bf16 *wb, bf16 *wt, float lr,
-                            float b1, float b2, float eps, float c1, float c2) {
+                            float b1, float b2, float eps, float c1, float c2, const int32_t *err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kMlpParams) return;
+  const int32_t failed = *err;
   int l = 0;
   while (l < 3 && i >= mlp_woff(l + 1)) l++;
   const int e = i - mlp_woff(l), K = mlp_K(l);
   const bool isb = i >= mlp_boff(l);
-  float gi = grad[i];
-  if (isb) grad[i] = gi = (float)gbias[l * kMlpW + i - mlp_boff(l)];
+  const float gi = isb ? (float)gbias[l * kMlpW + i - mlp_boff(l)] : grad[i];
   const float mi = b1 * m[i] + (1.f - b1) * gi, vi = b2 * v[i] + (1.f - b2) * gi * gi;
+  const float x = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  if (failed) return;
+  if (isb) grad[i] = gi;
   m[i] = mi;
   v[i] = vi;
-  const float x = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   w[i] = x;
   if (!isb) {
     const bf16 b = __float2bfloat16_rn(x);
@@ -1469,13 +1472,13 @@ int mlp_train_step(MlpParams &m, const bf16 *X, const float *T, const int32_t *r
   }
   double *gbias = reinterpret_cast<double *>(m.grad + kMlpGradBias);
   cudaMemsetAsync(m.grad, 0, kMlpGradBytes, s);
-  MlpTrainK p{X, T, rows, batch, m.wb, m.wt, m.master, m.grad, gbias, loss, m.err};
+  MlpTrainK p{X, T, rows, batch, m.wb, m.wt, m.master, m.grad, gbias, loss, m.err + kMlpErrTrain};
   k_mlp_train<<<(batch + kTcRows - 1) / kTcRows, kTrThreads, kTrSmem, s>>>(p);
   m.step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - powf(b1, (float)m.step), c2 = 1.f - powf(b2, (float)m.step);
   k_adam_pack<<<(kMlpParams + 255) / 256, 256, 0, s>>>(m.master, m.grad, gbias, m.mom, m.vel, m.wb, m.wt, lr, b1, b2,
-                                                      1e-8f, c1, c2);
+                                                      1e-8f, c1, c2, m.err + kMlpErrTrain);
   return cudaGetLastError() == cudaSuccess ? CUBE_OK : CUBE_ERR_CUDA;
 }
 

@@ -296,7 +296,8 @@ typedef struct cube_mlp cube_mlp;
 /* Upload the parameters; training steps take at most batch_cap rows (a multiple of 16). */
 int cube_mlp_create(const float *params, int32_t batch_cap, cube_mlp **mlp);
 int cube_mlp_destroy(cube_mlp *mlp);
-/* Current parameters and the gradients of the last training step (either may be NULL). */
+/* Current parameters and the gradients of the last training step (either may be NULL).  CUBE_ERR_TIMEOUT after a
+ * training step whose bounded wait ran out: the parameters are those before it, and later steps change nothing. */
 int cube_mlp_get_params(cube_mlp *mlp, float *params, float *grads);
 /* Input rows d_X (BF16 [n_used][80], zeros for buffer copies) of every stored copy of the
  * image, in storage order (the training input). */
