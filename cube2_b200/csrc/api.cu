@@ -607,9 +607,10 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
       launch_pm3_force(a, g.stream);
       g.launches += 1;
     }
-    auto gather = [&](const PM3Args &ga) {
-      if (fused) launch_pm3_force_gather(ga, g.stream);
-      else launch_pm3_gather(ga, g.stream);
+    auto gather = [&](const PM3Args &ga) {  // false: not launched
+      if (fused) return launch_pm3_force_gather(ga, g.stream);
+      launch_pm3_gather(ga, g.stream);
+      return true;
     };
     if (g.vp_pending && g.vp_tiles == g.ngrp && g.ngrp > 0) {  // gather each group once its vp is in
       PM3Args at = a;
@@ -619,7 +620,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
         at.jobs = (const MeshJob *)g.jobs.p + g.grp_lo[k];
         at.njobs = g.grp_lo[k + 1] - g.grp_lo[k];
         at.brick_ctr = a.brick_ctr + k;
-        gather(at);
+        if (!gather(at)) return fail(CUBE_ERR_CUDA);
         CU(cudaEventRecord(g.ev_ready[k], g.stream));
       }
       g.vp_pending = false;
@@ -627,7 +628,7 @@ static int run_pm3(const Meta &m, const int32_t *ires, const int32_t *ratio_sf, 
       g.launches += g.ngrp - 1;
     } else {
       CK(wait_vp());
-      gather(a);
+      if (!gather(a)) return fail(CUBE_ERR_CUDA);
     }
     g.launches += 1;
     CU(cudaGetLastError());

@@ -292,7 +292,7 @@ void launch_pm3_gather(const PM3Args &a, cudaStream_t s);
 // at least four buffer points per side
 int pm3_brick_mc(const PM3Args &a);
 int64_t pm3_deposit_bricks(const PM3Args &a);  // bricks of the deposited cells (0: the geometry does not apply)
-bool launch_pm3_force_gather(const PM3Args &a, cudaStream_t s);  // reads a.phi
+[[nodiscard]] bool launch_pm3_force_gather(const PM3Args &a, cudaStream_t s);  // reads a.phi
 void launch_pm3_ghosts(const PM3Args &a, cudaStream_t s);          // fills the ghost points of a.phi
 void launch_green_fp64(int n, double apm_soft, double apm_range, double gridsize, int p_order, float *G,
                        cudaStream_t s);
