@@ -2071,8 +2071,12 @@ int cube_mlp_kick(cube_mlp *h, const int32_t *d_rhoc, const int64_t *d_idx_b_r, 
   CK(ensure_device());
   const StreamScope scope(stream);
   cudaStream_t s = g.stream;
-  CK(grow(g.mlp_tab, sizeof(uint2) * (size_t)g.L.ng * g.L.ng * g.L.ng));
   CK(mlp_density(d_rhoc, d_idx_b_r, d_xp, n_used, true));
+  // without memory for the table the network reads the density itself
+  if (grow(g.mlp_tab, sizeof(uint2) * (size_t)g.L.ng * g.L.ng * g.L.ng) != CUBE_OK) {
+    cudaGetLastError();
+    t_last_error = CUBE_OK;
+  }
   // the kick coefficient of run_kick (kick.f90:529), times the network's output scale
   const float kick = (float)((double)(a_mid * dt / 6.0f) / 3.14159265358979323846);
   launch_mlp_apply(h->p, (const float4 *)g.mlp_pos.p, (const unsigned long long *)g.mlp_n.p, (float *)g.mlp_rho.p,

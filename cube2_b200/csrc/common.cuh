@@ -405,7 +405,8 @@ void launch_mlp_list(const Lay &L, const int16_t *xp, const int32_t *rhoc, const
 void launch_mlp_cic(const float4 *list, const unsigned long long *n_list, int ng, float *rho, cudaStream_t s);
 void launch_mlp_log1p(float *rho, int64_t n, cudaStream_t s);
 void launch_mlp_features(const float4 *pos, int64_t n, const float *rho, int ng, __nv_bfloat16 *X, cudaStream_t s);
-// the fused inference + kick on the density rho (two kernels; rho may be overwritten); tab: 8 bytes a fine cell of scratch
+// the fused inference + kick on the density rho (two kernels; rho may be overwritten); tab: 8 bytes a fine cell of
+// scratch, or null: the inference then gathers from the density itself (slower)
 void launch_mlp_apply(const MlpParams &m, const float4 *list, const unsigned long long *n_list, float *rho, void *tab,
                       int ng, float *vp, float coef, int num_sms, cudaStream_t s);
 void launch_mlp_pack(MlpParams &m, cudaStream_t s);

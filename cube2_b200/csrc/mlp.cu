@@ -443,8 +443,8 @@ struct MlpApplyK {
   const float *master;
   const float4 *list;  // interior copies: fine position, w = storage index
   const unsigned long long *n_list;
-  const float *rho;   // log(1 + density) per fine cell (k_mlp_apply)
-  const uint2 *tab;   // k_mlp_table's stencil rows (k_mlp_apply_tc)
+  const float *rho;   // log(1 + density) per fine cell (where tab is null, and in k_mlp_apply)
+  const uint2 *tab;   // k_mlp_table's stencil rows
   int ng;
   float *vp;
   float coef;  // kick coefficient times the output scale
@@ -719,10 +719,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
 
 // the inputs of mlp_inputs written straight into row m of the activation buffer, one 8-value
 // chunk at a time: chunk 2 dz + h holds the stencil rows dy = 2h - 1, 2h of plane dz (x fastest),
-// chunk 8 the offsets, chunk 9 zeros.  A row is one 8-byte load of the table (64 scattered 4-byte loads and
-// as many conversions a particle before: the kernel's L1 was 65 % busy with them)
-__device__ __forceinline__ void tc_inputs(float4 q, bool live, const uint2 *__restrict__ tab, int ng,
-                                          unsigned char *act, int m) {
+// chunk 8 the offsets, chunk 9 zeros.  TAB: a row is one 8-byte load of the table (64 scattered 4-byte loads of rho
+// and as many conversions a particle without it: the kernel's L1 was 65 % busy with them)
+template <bool TAB>
+__device__ __forceinline__ void tc_inputs(float4 q, bool live, const uint2 *__restrict__ tab, const float *__restrict__ rho,
+                                          int ng, unsigned char *act, int m) {
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   if (!live) {
 #pragma unroll
@@ -738,21 +739,42 @@ __device__ __forceinline__ void tc_inputs(float4 q, bool live, const uint2 *__re
     i0[d] = (int)fl;
     f[d] = xs[d] - fl;
   }
-  const uint2 *const col = tab + wrap_cell(wrap_cell(i0[0] - 1, ng), ng);
-  int Y[4];
+  int X[4], Y[4];
 #pragma unroll
-  for (int dy = 0; dy < 4; dy++) Y[dy] = wrap_cell(wrap_cell(i0[1] + dy - 1, ng), ng);
-  uint2 v[16];
-#pragma unroll
-  for (int dz = 0; dz < 4; dz++) {
-    const int64_t Z = wrap_cell(wrap_cell(i0[2] + dz - 1, ng), ng);
-#pragma unroll
-    for (int dy = 0; dy < 4; dy++) v[4 * dz + dy] = __ldg(col + (Z * ng + Y[dy]) * ng);
+  for (int d = 0; d < 4; d++) {
+    X[d] = wrap_cell(wrap_cell(i0[0] + d - 1, ng), ng);
+    Y[d] = wrap_cell(wrap_cell(i0[1] + d - 1, ng), ng);
   }
+  if constexpr (TAB) {
+    const uint2 *const col = tab + X[0];
+    uint2 v[16];
 #pragma unroll
-  for (int c = 0; c < 8; c++)
-    *reinterpret_cast<uint4 *>(act + umma_off(m, 8 * c, kTcRows)) =
-        make_uint4(v[2 * c].x, v[2 * c].y, v[2 * c + 1].x, v[2 * c + 1].y);
+    for (int dz = 0; dz < 4; dz++) {
+      const int64_t Z = wrap_cell(wrap_cell(i0[2] + dz - 1, ng), ng);
+#pragma unroll
+      for (int dy = 0; dy < 4; dy++) v[4 * dz + dy] = __ldg(col + (Z * ng + Y[dy]) * ng);
+    }
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      *reinterpret_cast<uint4 *>(act + umma_off(m, 8 * c, kTcRows)) =
+          make_uint4(v[2 * c].x, v[2 * c].y, v[2 * c + 1].x, v[2 * c + 1].y);
+  } else {
+#pragma unroll 1
+    for (int dz = 0; dz < 4; dz++) {
+      const int64_t Z = wrap_cell(wrap_cell(i0[2] + dz - 1, ng), ng);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        __align__(16) __nv_bfloat162 v[4];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          const float *row = rho + (Z * ng + Y[2 * h + r]) * ng;
+          v[2 * r] = __floats2bfloat162_rn(__ldg(row + X[0]), __ldg(row + X[1]));
+          v[2 * r + 1] = __floats2bfloat162_rn(__ldg(row + X[2]), __ldg(row + X[3]));
+        }
+        *reinterpret_cast<uint4 *>(act + umma_off(m, 16 * dz + 8 * h, kTcRows)) = *reinterpret_cast<const uint4 *>(v);
+      }
+    }
+  }
   __align__(16) __nv_bfloat162 o[4];
   o[0] = __floats2bfloat162_rn(f[0], f[1]);
   o[1] = __floats2bfloat162_rn(f[2], 0.f);
@@ -782,6 +804,7 @@ __device__ __forceinline__ void tc_issue(uint32_t tmem_d, uint32_t a_base, uint3
   umma_commit(bar);
 }
 
+template <bool TAB>
 __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_apply_tc(MlpApplyK p, int32_t *err) {
   extern __shared__ __align__(1024) unsigned char tc_smem[];
   unsigned char *w1 = tc_smem, *w2 = tc_smem + kTcOffW2, *w3 = tc_smem + kTcOffW3, *w4 = tc_smem + kTcOffW4;
@@ -828,7 +851,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_apply_tc(MlpApplyK p, int
     const int64_t i = tile * kTcRows + m;
     const bool live = i < n;
     const float4 q = live ? p.list[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    tc_inputs(q, live, p.tab, p.ng, act, m);  // layer-1 input row of this particle
+    tc_inputs<TAB>(q, live, p.tab, p.rho, p.ng, act, m);  // layer-1 input row of this particle
     // layers 1-3 (N = 128): MMA, then bias + GELU + BF16 back into the activation buffer
 #pragma unroll 1
     for (int l = 0; l < 3 && ok; l++) {
@@ -1396,17 +1419,21 @@ void launch_mlp_apply(const MlpParams &m, const float4 *list, const unsigned lon
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(k_mlp_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kApplySmem);
-    cudaFuncSetAttribute(k_mlp_apply_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
+    cudaFuncSetAttribute(k_mlp_apply_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
+    cudaFuncSetAttribute(k_mlp_apply_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
     attr = true;
   }
   MlpApplyK p{m.wb, m.master, list, n_list, rho, (const uint2 *)tab, ng, vp, coef};
   if (getenv("CUBE_MLP_MMA_SYNC")) {
     launch_mlp_log1p(rho, (int64_t)ng * ng * ng, s);
     k_mlp_apply<<<num_sms, kApplyWarps * 32, kApplySmem, s>>>(p);
+  } else if (!tab) {
+    launch_mlp_log1p(rho, (int64_t)ng * ng * ng, s);
+    k_mlp_apply_tc<false><<<num_sms, kTcThreads, kTcSmem, s>>>(p, m.err);
   } else {
     const dim3 grid((unsigned)((ng + kTabCells - 1) / kTabCells), (unsigned)ng, (unsigned)ng);
     k_mlp_table<<<grid, kTabCells, 0, s>>>(rho, ng, (uint2 *)tab);
-    k_mlp_apply_tc<<<num_sms, kTcThreads, kTcSmem, s>>>(p, m.err);
+    k_mlp_apply_tc<true><<<num_sms, kTcThreads, kTcSmem, s>>>(p, m.err);
   }
 }
 
