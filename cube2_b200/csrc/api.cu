@@ -2068,6 +2068,7 @@ int cube_mlp_kick(cube_mlp *h, const int32_t *d_rhoc, const int64_t *d_idx_b_r, 
   t_last_error = CUBE_OK;
   if (!g.configured) return fail(CUBE_ERR_NOT_CONFIGURED);
   if (!h || !d_rhoc || !d_idx_b_r || !d_xp || !d_vp || n_used < 0) return fail(CUBE_ERR_INVALID);
+  if (n_used >= ((int64_t)1 << 32)) return fail(CUBE_ERR_INVALID);  // the listed copies' storage indices
   CK(ensure_device());
   const StreamScope scope(stream);
   cudaStream_t s = g.stream;

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_mlp_pos(MlpPosK p) {
 }
 
 // The interior copies alone, as a list: a block takes 32 physical coarse cells, reserves their places with
-// one atomic and writes fine position and storage index (w).  The order of the list does not matter to
+// one atomic and writes fine position and storage index (w, below 2^32).  The order of the list does not matter to
 // the kick (every particle's output depends on its own inputs only).  The position is the one of
 // k_mlp_pos: c ratio_cs and (2u + 1) ratio_cs / 2^17 are exact in FP32, so their sum rounds once.
 constexpr int kListCells = 32;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_mlp_list(MlpListK p) {
 #pragma unroll
       for (int d = 0; d < 3; d++)
         if (v[d] >= (float)p.ng) v[d] = 0.f;
-      dst[l] = make_float4(v[0], v[1], v[2], __int_as_float((int)(base + l)));
+      dst[l] = make_float4(v[0], v[1], v[2], __uint_as_float((unsigned)(base + l)));
     }
   }
 }
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, 1) k_mlp_apply(MlpApplyK p) 
       for (int h = 0; h < 2; h++) {
         const int64_t i = r0 + g + 8 * h;
         if (i >= n) continue;
-        float *v = p.vp + 3 * (int64_t)__float_as_int(p.list[i].w) + 2 * t;
+        float *v = p.vp + 3 * (int64_t)__float_as_uint(p.list[i].w) + 2 * t;
         v[0] += p.coef * (acc[2 * h] + bias[3 * kMlpW + 2 * t]);
         if (t == 0) v[1] += p.coef * (acc[2 * h + 1] + bias[3 * kMlpW + 1]);
       }
@@ -901,7 +901,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_apply_tc(MlpApplyK p, int
     float y[4];
     tmem_ld4(tmem + lane_base, y);
     if (live) {
-      float *v = p.vp + 3 * (int64_t)__float_as_int(q.w);
+      float *v = p.vp + 3 * (int64_t)__float_as_uint(q.w);
       v[0] += p.coef * (y[0] + bias[3 * kMlpW + 0]);
       v[1] += p.coef * (y[1] + bias[3 * kMlpW + 1]);
       v[2] += p.coef * (y[2] + bias[3 * kMlpW + 2]);
