@@ -390,6 +390,8 @@ def run_ours(args, rank, world, local_rank):
     elif rank == 0 and world == 1 and not args.no_cpu_baseline:
         try:
             cpu = cpu_reference(args.workload, img)
+        except FileNotFoundError:
+            cpu = {"unavailable": NOT_BUILT}
         except Exception as e:  # the baseline must not hide our number
             cpu = {"error": repr(e)}
 
@@ -733,6 +735,8 @@ def per_box_loop(workload: str, fk_batch, img, stream, a_mid, dt, ms_batched):
 # ------------------------------------------------------------------------------------------------
 # reference CPU path (the baseline leg and the reference arm)
 
+NOT_BUILT = "the reference's PP kernel is compiled from its sources (oracle/build_ref.py), which are not on this machine"
+
 
 def _nnest_for_host():
     n = os.cpu_count() or 1
@@ -961,7 +965,11 @@ def run_reference(args, rank, world):
                           "workloads; batch workloads compare against a per-box launch loop instead"}))
         return
     img = W.make(args.workload)
-    setup = reference_setup(args.workload, img)
+    try:
+        setup = reference_setup(args.workload, img)
+    except FileNotFoundError:
+        print(json.dumps({"impl": "reference", "unavailable": NOT_BUILT}))
+        return
     pp, pm3 = [], []
     for s in range(args.warmup + args.steps):
         t_pp, t_pm3 = reference_step(args.workload, img, setup)
