@@ -117,7 +117,8 @@ def features(layout: Layout, d_rhoc, d_idx, d_xp, n_used: int, stream=None):
     import torch
     X = torch.zeros((max(n_used, 1), K_PAD), dtype=torch.bfloat16, device=d_xp.device)
     FineKick(layout, pm3_mode=CUBE_PM3_PERIODIC)
-    torch.cuda.current_stream(d_xp.device).synchronize()  # X is zero before the rows are written
+    if stream is None:
+        torch.cuda.current_stream(d_xp.device).synchronize()  # X is zero before the rows are written
     _check(lib().cube_mlp_features(_dp(d_rhoc), _dp(d_idx), _dp(d_xp), ctypes.c_int64(n_used), _dp(X),
                                    _sp(stream)), "cube_mlp_features")
     if stream is None:
