@@ -44,11 +44,11 @@ if ROOT not in sys.path:
 METRIC = "particle kicks/s (PM3+PP) on 1 B200, learned vs plain at equal rms force error"
 UNIT = "particle-kicks/s"
 PP_FLOP_PER_PAIR = 38  # 3 sub, 5 r^2, rsqrt, 1/r^2, 2 ep, 18 polynomial+reciprocal, 1 diff, 1 scale, 6 accumulate
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_pp_force launch per stored
-# particle, from an ncu capture on clustered192 (242.6 MB + 65.1 MB over 9,025,370 stored
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_pp_pairs launch per stored
+# particle, from an ncu capture on clustered192 (241 MB + 65 MB over 9,025,370 stored
 # particles); the kernel streams the sorted particles and vp once per launch, so the figure is
 # scaled to a full launch by the stored particle count
-PP_DRAM_BYTES_PER_STORED = (242_559_488 + 65_138_432) / 9_025_370
+PP_DRAM_BYTES_PER_STORED = (241e6 + 65e6) / 9_025_370
 
 
 def parse():
@@ -330,7 +330,7 @@ def run_ours(args, rank, world, local_rank):
                 "peak_source": "FP32 FMA probe measured in this run (MEASURED_PEAKS.json has no FP32 figure)",
                 "flops_per_launch": int(flops), "pairs_per_launch": int(pairs),
                 "traffic": float(PP_DRAM_BYTES_PER_STORED * img.n_used),
-                "traffic_source": "ncu DRAM bytes of k_pp_force on clustered192, scaled by stored particles"}
+                "traffic_source": "ncu DRAM bytes of k_pp_pairs on clustered192, scaled by stored particles"}
 
     # the whole kick against its roofline model: algorithmic bytes B = 64 B per particle + 66 B per
     # mesh point (binning 16, deposit 6, PP 12, gather 6, velocity 24 B per particle; deposit 4,

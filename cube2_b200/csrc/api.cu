@@ -2112,7 +2112,8 @@ int cube_kick_graph_create(const int32_t *isort, const int32_t *ires, const int3
   if (!out) return fail(CUBE_ERR_INVALID);
   *out = nullptr;
   if (!g.configured) return fail(CUBE_ERR_NOT_CONFIGURED);
-  // the subtile geometry synchronises the host between mesh batches, which a graph cannot hold
+  // The subtile geometry is refused, as it was when its mesh batches waited on the host; its kick takes Green tables
+  // from the caller, for which this call has no argument
   if (g.L.pm3_mode == CUBE_PM3_SUBTILE) return fail(CUBE_ERR_INVALID);
   if (!apm3 || !d_rhoc || !d_idx_b_r || !d_out || (n_used > 0 && (!d_xp || !d_vp))) return fail(CUBE_ERR_INVALID);
   if (n_used < 0 || n_used >= ((int64_t)1 << 31)) return fail(CUBE_ERR_INVALID);

@@ -279,7 +279,8 @@ int launch_pm3_deposit(const PM3Args &a, cudaStream_t s);  // returns the kernel
 // CIC instead of TSC on the brick kernels' geometry (pm3_brick_mc != 0, else nothing and 0): cell-centred points
 int launch_cic_bricks(const PM3Args &a, cudaStream_t s);
 void launch_pm3_kspace(const PM3Args &a, cudaStream_t s);
-void set_smem_attr_once(const void *fn, size_t bytes);  // dynamic shared-memory limit, raised once per device
+// dynamic shared-memory limit, raised once per device.  Its table has no lock of its own: called under the entry points' lock
+void set_smem_attr_once(const void *fn, size_t bytes);
 // Density to potential in this library's own transforms (mesh sides where pm3_fft_ok): a.rho to a.phi, with
 // ghost points where a.phi_pad > 0, or in place without a.phi.  Returns the kernels it launched
 bool pm3_fft_ok(int n, int nslots);

@@ -6,16 +6,17 @@
 namespace cube {
 
 // ---------------------------------------------------------------------------------------------
-// The potential's transforms on mesh sides 16 m of 64 to 1024 points with factors 2, 3 and 5, five passes over the mesh:
+// The potential's transforms on 19 mesh sides of 64 to 1024 points (CUBE_FFT_SIDES), five passes over the mesh:
 //   k_fft_rows      real rows along x to half spectra, [z][ky][kx], rows padded to whole 32-byte sectors;
 //   k_fft_columns   along y;
 //   k_fft_columns   along z, times the Green table (real), and back along z;
 //   k_fft_columns   back along y;
 //   k_ifft_rows     back along x, into the padded potential, ghost points included.
 // Every pass is one read and one write of the spectrum and is bound by that: no pass does more than about 4
-// operations a byte.  At 512^3 points (us): 210, 256, 425, 254, 222 against 313, 226, 439, 226, 344 + 34 for the ghost
-// points with cuFFT's plane transforms; at 1024^3 (ms) 1.78, 2.36, 4.32, 2.36, 1.99 against 1.57, 2.21, 6.07, 2.21,
-// 2.67 + 0.13; 64 meshes of 64^3: 171 against 255 us.  4 to 5 TB/s where a pass follows the rows; along z the
+// operations a byte.  At 512^3 points (us): 226, 256, 425, 255, 221 against 313, 226, 439, 226, 344 + 34 for the ghost
+// points with cuFFT's plane transforms; at 1024^3 (ms) 1.91, 2.38, 4.30, 2.38, 1.98 against 1.57, 2.21, 6.07, 2.21,
+// 2.67 + 0.13; 64 meshes of 64^3: 166 against 255 us.  (Rows of a power of two were at 210 us and 1.78 ms before the
+// passes of radix 5 and 3 came into the same source: 32 bytes of spills at 512 points.)  4 to 5 TB/s where a pass follows the rows; along z the
 // 64-byte pieces of a column lie a plane apart and it is 2.6 to 3.2 TB/s.
 // Sides with factors 3 and 5, where cuFFT transformed whole meshes around a separate Green multiply: the kick of a
 // 120^3 box (240^3 points) 1090 -> 990 us, of the subtile meshes of a 128^3 box (80^3 points) 2724 -> 2605 us.
@@ -459,8 +460,10 @@ __global__ void __launch_bounds__(ColFft<N>::T, ColFft<N>::kBlocks)
   }
 }
 
-// Mesh sides of the own transforms: 64 to 1024, multiples of 16 (eight points of a row's half transform a thread) with
-// factors 2, 3 and 5.  cuFFT's three-dimensional transforms serve the others.
+// Mesh sides of the own transforms: multiples of 16 (eight points of a row's half transform a thread) with factors 2, 3
+// and 5, those of the workloads, of the tests and between them.  It is a selection: the passes could be
+// instantiated for 400, 432, 720, 800 and 864 points too, which are neither built nor measured.  cuFFT's
+// three-dimensional transforms serve these and all other sides, those below 64 points among them.
 #define CUBE_FFT_SIDES(X) \
   X(64) X(80) X(96) X(128) X(144) X(160) X(192) X(240) X(256) X(288) X(320) X(384) X(480) X(512) X(576) X(640) X(768) X(960) X(1024)
 bool pm3_fft_ok(int n, int nslots) {

@@ -7,14 +7,15 @@
 // of the CIC density of all particles on the 4^3 fine cells i0-1 .. i0+2 around
 // i0 = floor(x - 0.5) (x fastest), then the offsets x - 0.5 - i0: 67 values, padded to 80.
 // Network: 67 -> 128 -> 128 -> 128 -> 3, tanh-GELU, BF16 operands on the tensor cores
-// (mma.sync m16n8k16, FP32 accumulation), FP32 biases and FP32 master weights for Adam.
+// (FP32 accumulation), FP32 biases and FP32 master weights for Adam.
 //
-// Kernels: positions per stored particle, the CIC density, the feature rows (training
-// input), a generic C = A B^T GEMM with bias / GELU epilogue (training forward and
-// backward, K a multiple of 16), GELU backward, column sums, transposes, the MSE loss,
-// Adam, and the fused inference kernel of the kick: every warp takes 16 particles through
-// all four layers with the weights resident in shared memory and adds the predicted force
-// times the kick coefficient to vp of the interior particles.
+// Kernels of the path (tcgen05, accumulators in tensor memory): the fused inference of the kick
+// (k_mlp_list, k_mlp_table, k_mlp_apply_tc: every warpgroup takes 128 particles through all four layers with the weights
+// resident in shared memory and adds the predicted force times the kick coefficient to vp), a training
+// step (k_mlp_train, k_adam_pack) and the GEMM of the forward pass (k_gemm_nt_tc).  Positions, feature rows (training
+// input) and the CIC density by particle are plain kernels.
+// CUBE_MLP_MMA_SYNC selects the form the path had before, kept as an independent check: mma.sync m16n8k16, a training
+// step as separate GEMMs, GELU backward, column sums, transposes, loss and Adam.
 #include <algorithm>
 #include <cstdlib>
 

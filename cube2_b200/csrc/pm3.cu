@@ -1004,7 +1004,8 @@ int pm3_brick_mc(const PM3Args &a) {
   return a.n >= 16 && a.n % 4 == 0 && a.shift % 4 == 0 ? mc : 0;
 }
 
-// the dynamic shared-memory limit of a kernel, raised once per device (the attribute is per device)
+// the dynamic shared-memory limit of a kernel, raised once per device (the attribute is per device).  Like the other
+// tables of this kind (tensor_map_encoder, the attributes in mlp.cu) it relies on the lock that every entry point holds
 void set_smem_attr_once(const void *fn, size_t bytes) {
   constexpr int kDev = 64, kFn = 96;
   static const void *fns[kFn] = {};

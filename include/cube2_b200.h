@@ -270,7 +270,9 @@ typedef struct cube_pp_shape_info {
   int32_t chunk, jtile, unroll, blocks, packed;
   float ms; /* the last tuning's time of the shape (work list + force kernel), -1 if never timed */
 } cube_pp_shape_info;
-/* shape >= 0: use that shape for every PP kick; -1: autotune (default; forgets earlier picks). */
+/* shape >= 0: use that shape for every PP kick; -1: autotune (default; forgets earlier picks).  Shapes are numbered by
+ * the table that cube_pp_shapes returns, whose size and order belong to the build: look a shape up there.  A number
+ * outside the table is CUBE_ERR_INVALID. */
 int cube_pp_set_shape(int32_t shape);
 /* The shape table (up to `cap` entries), its size and the shape of the last PP kick. */
 int cube_pp_shapes(cube_pp_shape_info *out, int32_t cap, int32_t *n_shapes, int32_t *current);
