@@ -118,6 +118,7 @@ struct Ctx {
   Buf fb_out;                  // learned-shell fallback statistics
   Buf phi_pad;                 // padded potential of the brick kernels
   Buf dep_items;               // the brick deposit's work list
+  Buf pm_items;                // and PM2's
   cudaEvent_t tune_ev[2 * kMaxPPShapes] = {};
   void *h_stage = nullptr;  // pinned staging for small tables
   size_t h_stage_cap = 0;
@@ -1488,10 +1489,11 @@ static int run_pm_layer(int layer, const Dev &d, float mass, float kick, float a
   a.vp = d.vp;
   a.out = (float *)g.out.p;
   a.want_vmax = 1;
-  // Crowded bricks in pieces, as in the kick: without the list one block walks a brick however many particles it
-  // holds, and its fixed-point scale falls with their number (2^16 at 10^5)
-  CK(grow(g.dep_items, pm3_dep_items_bytes((int64_t)a.rdep[0] * a.rdep[1] * a.rdep[2], a.njobs, d.n_used)));
-  a.dep_items = (int2 *)g.dep_items.p;
+  // Crowded bricks in pieces, as in the kick: without a list one block walks a brick however many particles it holds, and
+  // its fixed-point scale falls with their number (2^16 at 10^5).  The list is longer than the kick's, which a
+  // captured graph keeps the place of: it has its own buffer
+  CK(grow(g.pm_items, pm3_dep_items_bytes((int64_t)a.rdep[0] * a.rdep[1] * a.rdep[2], a.njobs, d.n_used)));
+  a.dep_items = (int2 *)g.pm_items.p;
   a.n_particles_hint = d.n_used;
   const bool own = pm3_fft_ok(n, nslots);
   cufftHandle fw = 0, bw = 0;
@@ -2234,6 +2236,7 @@ void c_pm3_fft_finalize(void) {
   release(g.force);
   release(g.phi_pad);
   release(g.dep_items);
+  release(g.pm_items);
   release(g.jobs);
   release(g.mlp_pos);
   release(g.mlp_rho);
